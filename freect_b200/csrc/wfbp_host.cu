@@ -171,6 +171,8 @@ void release(wfbp_ctx* ctx) {
   free_dev(ctx->d_fuse_slab_tab);
   free_dev(ctx->d_fuse_tab);
   free_dev(ctx->d_bplanes);
+  free_dev(ctx->d_fft_tw);
+  free_dev(ctx->d_fft_spec);
   free_dev(ctx->d_err);
   free_dev(ctx->d_thickT_off);
   free_dev(ctx->d_thickT_idx);
@@ -724,6 +726,12 @@ WFBP_API int wfbp_ctx_create(const CTGeometry* cg, const ReconConfig* rp, const 
     }
     if (!ce) ce = alloc_copy((void**)&ctx->d_chan64, ch.data(), sizeof(double2) * nch);
   }
+  if (!ce && e.precision == WFBP_PRECISION_FP32 && (ctx->fft_n = filter_fft_size(ctx->nch)) > 0) {
+    std::vector<float2> tw(ctx->fft_n);
+    filter_fft_twiddles(ctx->fft_n, tw.data());
+    ce = alloc_copy((void**)&ctx->d_fft_tw, tw.data(), sizeof(float2) * ctx->fft_n);
+    if (!ce) ce = alloc_copy((void**)&ctx->d_fft_spec, nullptr, sizeof(float2) * ctx->fft_n);
+  }
   if (!ce) ce = launch_rebin_tables(ctx->d_chan_beta, ctx->d_chan_bidx, ctx->nch, cg->detector_central_col,
                                     cg->detector_pixel_size_col, cg->distance_source_to_detector, 0);
   if (!ce) ce = cudaDeviceSynchronize();
@@ -997,6 +1005,30 @@ WFBP_API int wfbp_rebin(wfbp_ctx* ctx, const float* raw, void* rebinned, void* s
 
 namespace {
 
+// FP32 filter of `rows` rows: by FFT (k_filter_fft.cu) where its transforms
+// take the channels (up to 2047), 6 to 9 times faster than the Toeplitz
+// product (k_toeplitz_f32) on scans of 96 to 1472 channels. A call computes the
+// taps' spectrum, since they may have changed (wfbp_set_taps); the later view
+// ranges of one pipelined run (spectrum = false) share it.
+// The forward filter of a context whose taps are being learned (wfbp_set_taps)
+// stays a Toeplitz product: the taps' gradient is a small difference of large
+// sums (the unfiltered backprojection times the image's residual), which a
+// change of 1e-8 in the filter's gain at zero frequency moves by 1e-4; the
+// adjoint filter enters only the readings' gradient.
+int filter_rows_f32(wfbp_ctx* ctx, const float* x, float* y, long rows, bool bpl, bool fft, bool spectrum,
+                    cudaStream_t s) {
+  if (ctx->fft_n && fft) {
+    if (spectrum) CUDA_TRY(ctx, launch_filter_spectrum(ctx->d_taps, ctx->nch, ctx->fft_n, ctx->d_fft_spec, s));
+    CUDA_TRY(ctx, launch_filter_fft(x, y, ctx->d_taps, ctx->d_fft_spec, ctx->d_fft_tw, ctx->fft_n, rows, ctx->nch,
+                                    ctx->nr, ctx->bpt.nrp, bpl, s));
+  } else if (bpl) {
+    CUDA_TRY(ctx, launch_filter_f32_tr(x, y, ctx->d_taps, rows, ctx->nch, ctx->nr, ctx->bpt.nrp, s));
+  } else {
+    CUDA_TRY(ctx, launch_filter_f32(x, y, ctx->d_taps, rows, ctx->nch, s));
+  }
+  return WFBP_OK;
+}
+
 // publish: write the FP16 pairs' scale into scales[vb..ve) (the stage API's
 // contract); the context's own runs skip it, their backprojection applies
 // the context's scale directly.
@@ -1035,14 +1067,8 @@ int do_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* scales
     return WFBP_OK;
   }
   const float* x = (const float*)rebinned + (size_t)vb * ctx->nr * ctx->nch;
-  const long rows = (long)(ve - vb) * ctx->nr;
-  if (bpl)
-    CUDA_TRY(ctx, launch_filter_f32_tr(x, (float*)filtered + (size_t)vb * ctx->nch * ctx->bpt.nrp, ctx->d_taps, rows,
-                                       ctx->nch, ctx->nr, ctx->bpt.nrp, s));
-  else
-    CUDA_TRY(ctx, launch_filter_f32(x, (float*)filtered + (size_t)vb * ctx->nr * ctx->nch, ctx->d_taps, rows, ctx->nch,
-                                    s));
-  return WFBP_OK;
+  float* y = (float*)filtered + (size_t)vb * ctx->nch * (bpl ? ctx->bpt.nrp : ctx->nr);
+  return filter_rows_f32(ctx, x, y, (long)(ve - vb) * ctx->nr, bpl, !ctx->taps_set, vb == 0, s);
 }
 
 int do_backproject(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol,
@@ -1117,6 +1143,7 @@ WFBP_API int wfbp_set_taps(wfbp_ctx* ctx, const float* taps, int n, void* stream
     return fail(ctx, WFBP_ERR_UNSUPPORTED, "wfbp_set_taps: the mixed form bakes its taps into the operand planes");
   DeviceGuard g(ctx->device);
   CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_taps, taps, sizeof(float) * n, cudaMemcpyDefault, (cudaStream_t)stream));
+  ctx->taps_set = true;
   return WFBP_OK;
 }
 
@@ -1184,9 +1211,7 @@ WFBP_API int wfbp_filter_adjoint(wfbp_ctx* ctx, const float* g_filtered, float* 
   if (st) return st;
   DeviceGuard g(ctx->device);
   // the Toeplitz operator h[|n - m|] is symmetric: its transpose is itself
-  CUDA_TRY(ctx, launch_filter_f32(g_filtered, g_rebinned, ctx->d_taps, (long)ctx->V * ctx->nr, ctx->nch,
-                                  (cudaStream_t)stream));
-  return WFBP_OK;
+  return filter_rows_f32(ctx, g_filtered, g_rebinned, (long)ctx->V * ctx->nr, false, true, true, (cudaStream_t)stream);
 }
 
 WFBP_API int wfbp_rebin_adjoint(wfbp_ctx* ctx, const float* g_rebinned, float* g_raw, void* stream) {

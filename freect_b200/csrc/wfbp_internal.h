@@ -184,6 +184,12 @@ struct wfbp_ctx {
   void* d_bplanes = nullptr;        // FP16 [2][tc_np][tc_kp] (hi, lo of tap_scale * T)
   int* d_err = nullptr;             // device-side error word (WFBP_ERR_TIMEOUT, or WFBP_ERRBIT_* bits)
 
+  // FP32 form's FFT filter (fft_n = 0: more channels than its largest transform takes)
+  int fft_n = 0;                    // transform length > 2 nch
+  float2* d_fft_tw = nullptr;       // [fft_n] exp(-2 pi i j / fft_n)
+  float2* d_fft_spec = nullptr;     // [fft_n] spectrum of the taps' running sums / fft_n, written by each filter call
+  bool taps_set = false;            // wfbp_set_taps was called: the forward filter stays the Toeplitz product
+
   // TMA-staged backprojection (backprojection layout [V][nch][nrp])
   bool bp_tma_ok = false;
   BPTile bpt;
@@ -250,6 +256,13 @@ cudaError_t launch_filter_tc(const void* a_planes, const void* b_planes, int M, 
                              const TcOutArgs& out, int* err, cudaStream_t s, int mb = 0, int me = -1);
 cudaError_t launch_filter_f32_tr(const float* x, float* yt, const float* d_taps, long rows, int nch, int nr, int nrp,
                                  cudaStream_t s);
+// FFT form of the FP32 filter (k_filter_fft.cu): transform length for nch
+// channels (0: none), its twiddles, the taps' spectrum, the filter itself
+int filter_fft_size(int nch);
+void filter_fft_twiddles(int N, float2* tw);
+cudaError_t launch_filter_spectrum(const float* d_taps, int nch, int N, float2* spec, cudaStream_t s);
+cudaError_t launch_filter_fft(const float* x, float* y, const float* d_taps, const float2* spec, const float2* tw, int N,
+                              long rows, int nch, int nr, int nrp, bool transposed, cudaStream_t s);
 // Thickening fused into the TMA backprojection's write-back: a requested
 // slice whose native slices (the thickening CSR row) all lie in one slab is
 // formed from that slab's registers and written to `out`; the other
