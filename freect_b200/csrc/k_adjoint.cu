@@ -10,6 +10,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 #include "bp_math.cuh"
 #include "rebin_sample.cuh"
 
@@ -30,17 +32,9 @@ __device__ __forceinline__ float q_weight_fwd(float qh) {
 //   vol += dtheta / sum_k W_k * sum_k W_k * bilinear(D_j; p_idx_j, q_idx_j).
 // The gradient of one filtered sample D[j][r][c] is therefore
 //   sum over voxels of g_vol * dtheta * W_j / sum_k W_k * hat(p_idx_j - c) * hat_row,
-// where hat is the bilinear weight. Ownership: a CTA owns view j and a run of
-// AD_CH consecutive channels; thread c walks the voxels whose p_idx lies in
-// [c, c + 1) (a band one channel wide around a line through the image,
-// traversed along its longer axis), so every (voxel, view) pair is visited
-// by exactly one thread. For each such voxel it visits the slices inside the
-// view's cone, takes g_vol * dtheta / sum_k W_k from the scale table (or
-// recomputes sum_k W_k from the same expressions as the forward), and adds
-// the row contributions to two accumulators of its own in shared memory: one
-// for channel c (weight 1 - frac(p_idx)) and one for channel c + 1 (weight
-// frac(p_idx)). At the end channel c = own(c) + next(c - 1), in that order;
-// the CTA's first thread only supplies next(c0 - 1) for its neighbour.
+// where hat is the bilinear weight. k_bp_adjoint_band gathers it with the
+// weights dtheta / sum_k W_k in a table; where no table fits,
+// k_bp_adjoint_sums recomputes the sums.
 constexpr int AD_CH = 128;
 
 __device__ __forceinline__ float xcoord(const BPParams& p, int ix) {
@@ -51,21 +45,24 @@ __device__ __forceinline__ float ycoord(const BPParams& p, int iy) {
 }
 
 struct ViewGeo {
-  float zt, A, lt, inv, p_idx;  // lt = l_hat tan(cone), inv = 1 / lt
+  float zt, asn, A, lt, inv, p_idx;  // asn = asin(p_hat / R), A = z_rot / 2 pi asn, lt = l_hat tan(cone), inv = 1 / lt
   bool valid_p;
 };
 
 __device__ __forceinline__ ViewGeo view_geo(const BPParams& p, float x, float y, float2 sc, float zt) {
   ViewGeo g;
   g.zt = zt;
-  const float p_hat = x * sc.x - y * sc.y;
+  // roundings written out: a view's borderline samples must fall the same way
+  // in every kernel, whatever the compiler hoists
+  const float p_hat = fmaf(x, sc.x, -__fmul_rn(y, sc.y));
   // the forward's short forms (bp_math.cuh): hardware square root and
   // reciprocal, arcsine from its series
-  const float l_hat = bp_sqrt(p.R2 - p_hat * p_hat) - x * sc.y - y * sc.x;
-  g.A = p.zr2pi * bp_asin(p.rR * p_hat);
+  const float l_hat = fmaf(-y, sc.x, fmaf(-x, sc.y, bp_sqrt(fmaf(-p_hat, p_hat, p.R2))));
+  g.asn = bp_asin(p.rR * p_hat);
+  g.A = p.zr2pi * g.asn;
   g.lt = l_hat * p.tanc;
   g.inv = bp_rcp(g.lt);
-  g.p_idx = p.kp - (p_hat * p.ps + p.c0);
+  g.p_idx = p.kp - fmaf(p_hat, p.ps, p.c0);
   const float pf = floorf(g.p_idx);
   g.valid_p = pf >= 0.0f && ceilf(g.p_idx) <= p.ncm2;
   return g;
@@ -74,72 +71,257 @@ __device__ __forceinline__ ViewGeo view_geo(const BPParams& p, float x, float y,
 // Q weight of view geometry g at slice z (0 where the forward skips it).
 __device__ __forceinline__ float view_weight(const BPParams& p, const ViewGeo& g, float z, float* q_idx_out) {
   const float dz = z - g.zt;
-  const float qh = (dz + g.A) * g.inv;
-  const float q_idx = (qh + 1.0f) * p.hn;
+  const float qh = __fmul_rn(fmaf(p.zr2pi, g.asn, dz), g.inv);
+  const float q_idx = __fmul_rn(__fadd_rn(qh, 1.0f), p.hn);
   *q_idx_out = q_idx;
   const bool ok = g.valid_p && fabsf(dz) <= p.z_rot && q_idx >= 0.0f && q_idx <= p.nrm2;
   return ok ? q_weight_fwd(qh) : 0.0f;
 }
 
-// Weights G[t][y][x][s] = dtheta / sum_k W_k for each half-turn angle t
-// (0 where no half turn contributes, as the forward's NaN voxel has no
-// gradient), slices innermost with a stride of nzp = nz rounded up to 4: one
-// thread per (x, y) column and ZS slices, the weights summed in the
-// forward's order. They depend on the geometry alone (views, slices, grid),
-// so the context computes them once and every later gradient reuses them;
-// with the table the gather below needs one load instead of the other half
-// turns' geometry, and a voxel's slice run is one contiguous span.
-constexpr int AN_ZS = 8, AN_TX = 16, AN_TY = 8;
+// The views of one half-turn angle lie pi apart, so they cross the image along
+// the same axis: p_hat = x sin - y cos changes faster along x when
+// |sin| >= |cos|. That axis is the angle's inner axis u, the other v.
+__device__ __forceinline__ bool inner_is_x(float2 sc) { return fabsf(sc.x) >= fabsf(sc.y); }
 
-__global__ void __launch_bounds__(AN_TX * AN_TY)
-k_bp_adjoint_scale(float* __restrict__ G, const float2* __restrict__ view_sc,
-                   const float* __restrict__ view_z, const float* __restrict__ zslices, BPParams p, int nzp) {
-  const int ix = blockIdx.x * AN_TX + (threadIdx.x % AN_TX);
-  const int iy = blockIdx.y * AN_TY + (threadIdx.x / AN_TX);
-  const int s0 = blockIdx.z * AN_ZS;
-  if (ix >= p.nx || iy >= p.ny) return;
-  const float x = xcoord(p, ix), y = ycoord(p, iy);
-  const size_t plane = (size_t)p.nx * p.ny, vox = (size_t)iy * p.nx + ix;
-  const bool active = !(x * x + y * y > p.fov_half2);
-  float z[AN_ZS];
+// Weights G[t - t0][s][v][u] = dtheta / sum_k W_k of half-turn angles t0 .. (0
+// where no half turn contributes, as the forward's NaN voxel has no
+// gradient). A thread takes one voxel column and 32 slices of one angle, lanes
+// along u: it computes the column's geometry for the views whose cone reaches
+// the slices and sums the weights of every slice in the forward's order.
+constexpr int AN_WARPS = 8;
+
+__global__ void __launch_bounds__(AN_WARPS * 32)
+k_bp_adjoint_scale(float* __restrict__ G, const float2* __restrict__ view_sc, const float* __restrict__ view_z,
+                   const float* __restrict__ zslices, BPParams p, int t0, float reach, int nv_max) {
+  extern __shared__ float2 s_geo[];  // [nv_max][threads] (inv, asn); then float [nv_max] table positions, [32] slices
+  float2* geo = s_geo + threadIdx.x;
+  float* zts = reinterpret_cast<float*>(s_geo + (size_t)AN_WARPS * nv_max * 32);
+  float* zs = zts + nv_max;
+  const int lane = threadIdx.x % 32;
+  const int t = t0 + (int)blockIdx.y, s0 = blockIdx.z * 32, ns = min(32, p.nz - s0);
+  if (threadIdx.x < 32) zs[threadIdx.x] = __ldg(zslices + s0 + min((int)threadIdx.x, ns - 1));
+  __syncthreads();
+  float zmn = zs[min(lane, ns - 1)], zmx = zmn;
 #pragma unroll
-  for (int i = 0; i < AN_ZS; i++) z[i] = s0 + i < p.nz ? __ldg(zslices + s0 + i) : 0.0f;
-  for (int t = 0; t < p.P2; t++) {
-    float aw[AN_ZS];
-#pragma unroll
-    for (int i = 0; i < AN_ZS; i++) aw[i] = 0.0f;
-    if (active) {
-      for (int k = 0; k < p.K; k++) {
-        const int j = t + k * p.P2;
-        const float zt = __ldg(view_z + j);
-        const ViewGeo g = view_geo(p, x, y, __ldg(view_sc + j), zt);
-        if (!g.valid_p) continue;
-#pragma unroll
-        for (int i = 0; i < AN_ZS; i++) {
-          float qi;
-          aw[i] += view_weight(p, g, z[i], &qi);
-        }
-      }
+  for (int o = 16; o > 0; o >>= 1) {
+    zmn = fminf(zmn, __shfl_xor_sync(0xffffffffu, zmn, o));
+    zmx = fmaxf(zmx, __shfl_xor_sync(0xffffffffu, zmx, o));
+  }
+  const bool ux = inner_is_x(__ldg(view_sc + t));
+  const int nu = ux ? p.nx : p.ny;
+  const long plane = (long)p.nx * p.ny, col = (long)blockIdx.x * (AN_WARPS * 32) + threadIdx.x;
+  const int u = (int)(col % nu), v = (int)(col / nu);
+  const float x = xcoord(p, ux ? u : v), y = ycoord(p, ux ? v : u);
+  const bool active = col < plane && !(x * x + y * y > p.fov_half2);
+  int n = 0;
+  for (int k = 0; k < p.K; k++) {
+    const int j = t + k * p.P2;
+    const float zt = __ldg(view_z + j);
+    // beyond the cone's reach (or z_rot) of all these slices every weight is 0
+    if (zt < zmn - reach || zt > zmx + reach || n >= nv_max) continue;
+    const ViewGeo g = view_geo(p, x, y, __ldg(view_sc + j), zt);
+    // an invalid column: no row coordinate
+    geo[n * (AN_WARPS * 32)] = make_float2(g.inv, active && g.valid_p ? g.asn : __int_as_float(0x7fc00000));
+    if (threadIdx.x == 0) zts[n] = zt;
+    n++;
+  }
+  __syncthreads();
+  if (col >= plane) return;
+  float* out = G + ((size_t)blockIdx.y * p.nz + s0) * plane + col;
+  for (int i = 0; i < ns; i++, out += plane) {
+    const float z = zs[i];
+    float aw = 0.0f;
+    for (int a = 0; a < n; a++) {
+      const float2 ga = geo[a * (AN_WARPS * 32)];
+      const float dz = z - zts[a];
+      const float qh = __fmul_rn(fmaf(p.zr2pi, ga.y, dz), ga.x);
+      const float q_idx = __fmul_rn(__fadd_rn(qh, 1.0f), p.hn);
+      const bool ok = fabsf(dz) <= p.z_rot && q_idx >= 0.0f && q_idx <= p.nrm2;
+      aw += ok ? q_weight_fwd(qh) : 0.0f;
     }
-    float* out = G + ((size_t)t * plane + vox) * nzp + s0;
-#pragma unroll
-    for (int i = 0; i < AN_ZS; i++)
-      if (s0 + i < nzp) out[i] = s0 + i < p.nz && aw[i] > 0.0f ? p.dtheta * (1.0f / aw[i]) : 0.0f;
+    *out = aw > 0.0f ? p.dtheta * (1.0f / aw) : 0.0f;
   }
 }
 
-template <bool TABLE>
+// Gather with the weight table. A CTA owns one view and a run of CH channels
+// and visits the voxels whose p_idx lies in its channels (a band across the
+// image) or in the channel before them (whose voxels share their sample with
+// the run's first channel). Its warps take the image rows v in turn; lanes are
+// VL consecutive voxels u of the row inside the band, times 32 / VL shares of
+// the slices in the view's cone, which they walk together. A slice's
+// g_vol dtheta / sum_k W_k W_j goes to the rows r and r + 1 around its row
+// coordinate, weighted for the voxel's channel c (1 - frac(p_idx)) and for
+// c + 1 (frac(p_idx)), into the warp's own window [row][channel] of (c, c + 1)
+// sums in shared memory. Neighbouring voxels are p_step channels apart and
+// the shares' slices a share's length: with p_step > 1 and shares of a few
+// rows no two lanes write the same sums at a time, else lanes take turns. At
+// the end the warps' windows are added in a fixed order: no atomics, nothing
+// depends on scheduling. Weights and gradient are read along u in full lines,
+// the next slice's before this one's arithmetic. Bound by instruction issue.
+constexpr int AB_WARPS = 8;
+
+__global__ void __launch_bounds__(AB_WARPS * 32, 3)
+k_bp_adjoint_band(const float* __restrict__ gvol_x, const float* __restrict__ gvol_y, const float* __restrict__ G,
+                  float* __restrict__ gD, const float2* __restrict__ view_sc, const float* __restrict__ view_z,
+                  const float* __restrict__ zslices, BPParams p, float z0, float dzs, int t0, float reach, int CH) {
+  extern __shared__ float2 s_win[];  // [AB_WARPS][nr][CH + 1] (sum for c, sum for c + 1); then float [nz] slices
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int tl = blockIdx.y / p.K, j = t0 + tl + (blockIdx.y % p.K) * p.P2;
+  const int W = CH + 1, wsize = W * p.nr, c_base = blockIdx.x * CH - 1;  // channel of a window's first column
+  float* s_z = reinterpret_cast<float*>(s_win + (size_t)AB_WARPS * wsize);
+  const int win = warp * wsize;
+  for (int e = threadIdx.x; e < AB_WARPS * wsize; e += AB_WARPS * 32) s_win[e] = make_float2(0.0f, 0.0f);
+  for (int e = threadIdx.x; e < p.nz; e += AB_WARPS * 32) s_z[e] = __ldg(zslices + e);
+  __syncthreads();
+
+  const float zt = __ldg(view_z + j);
+  const float za0 = s_z[0], za1 = s_z[p.nz - 1];
+  if (!(zt < fminf(za0, za1) - reach || zt > fmaxf(za0, za1) + reach)) {  // else no slice is in the cone's reach
+    const float2 sc = __ldg(view_sc + j);
+    const bool ux = inner_is_x(__ldg(view_sc + t0 + tl));
+    const int nu = ux ? p.nx : p.ny, nv = ux ? p.ny : p.nx;
+    const size_t plane = (size_t)p.nx * p.ny;
+    const float* Gt = G + (size_t)tl * p.nz * plane;
+    const float* gv = ux ? gvol_x : gvol_y;
+    // p_idx in [c_base, c_base + CH + 1) <=> p_hat in this interval (widened
+    // by a rounding margin; the exact forward test below decides)
+    const float ph_a = (p.kp - p.c0 - ((float)c_base + (float)(CH + 1))) / p.ps,
+                ph_b = (p.kp - p.c0 - (float)c_base) / p.ps;
+    const float marg = 0.02f / p.ps + 1e-3f * p.fov / (float)p.nx;
+    const float plo = fminf(ph_a, ph_b) - marg, phi = fmaxf(ph_a, ph_b) + marg;
+    const float su = p.fov / (float)nu, num = 0.5f * ((float)nu - 1.0f);
+    // candidate ranges through reciprocals computed once: their rounding (a few
+    // 1e-5 mm) stays far inside the margin
+    const float r_sc = 1.0f / (ux ? sc.x : sc.y), r_s = 1.0f / su;
+    const float r_dzs = dzs != 0.0f ? 1.0f / dzs : 0.0f, top_q = p.nrm2 / p.hn - 1.0f;
+    // voxels a few lanes apart that are sure to lie in different channels
+    const float p_step = p.ps * su * fabsf(ux ? sc.x : sc.y);
+    // lanes per run of voxels: the split with the fewest instructions for the
+    // band's width, a run costing its geometry (about 110) and 40 a slice
+    int VL = 32;
+    {
+      const float width = fminf((float)W / p_step + 1.0f, (float)nu), slices = fminf((float)p.nr, (float)p.nz);
+      float best = 3.0e38f;
+      for (int l = 32; l >= 4; l >>= 1) {
+        const float cost = ceilf(width / (float)l) * (110.0f + 40.0f * ceilf(slices * (float)l / 32.0f));
+        if (cost < best) {
+          best = cost;
+          VL = l;
+        }
+      }
+    }
+    const int vl = lane & (VL - 1), share = lane / VL, shares = 32 / VL;
+    const int v_turns = min((int)ceilf(fminf(1.001f / p_step, 64.0f)), VL), v_turn = vl % v_turns;
+    const float r_hd = r_dzs / p.hn;
+
+    for (int v = warp; v < nv; v += AB_WARPS) {
+      const float cv = ux ? ycoord(p, v) : xcoord(p, v);
+      float a, b;
+      if (ux) {
+        a = (plo + cv * sc.y) * r_sc - p.x0;
+        b = (phi + cv * sc.y) * r_sc - p.x0;
+      } else {
+        a = (cv * sc.x - phi) * r_sc - p.y0;
+        b = (cv * sc.x - plo) * r_sc - p.y0;
+      }
+      const int u_lo = max(0, (int)floorf(fminf(a, b) * r_s + num));
+      const int u_hi = min(nu - 1, (int)ceilf(fmaxf(a, b) * r_s + num));
+      for (int u0 = u_lo; u0 <= u_hi; u0 += VL) {
+        const int u = u0 + vl;
+        const float x = ux ? xcoord(p, u) : cv, y = ux ? cv : ycoord(p, u);
+        const ViewGeo g = view_geo(p, x, y, sc, zt);
+        const float pf = floorf(g.p_idx), wp = g.p_idx - pf, h0 = 1.0f - wp;
+        const int c = (int)pf - c_base;
+        const bool own = u <= u_hi && !(x * x + y * y > p.fov_half2) && g.valid_p && c >= 0 && c <= CH;
+        // slices that can pass this view's tests: |z - zt| <= z_rot and q_idx in
+        // [0, nr - 2], a z interval around zt - A (evenly spaced slices lie
+        // within 1e-3 of a slice of z0 + s dzs)
+        const float za = zt - g.A - g.lt, zb = zt - g.A + top_q * g.lt;
+        const float zlo = fmaxf(fminf(za, zb), zt - p.z_rot), zhi = fminf(fmaxf(za, zb), zt + p.z_rot);
+        int s_lo = 0, s_hi = p.nz - 1;
+        if (dzs != 0.0f) {
+          const float fa = (zlo - z0) * r_dzs, fb = (zhi - z0) * r_dzs;
+          s_lo = max(0, (int)ceilf(fminf(fa, fb) - 0.01f));
+          s_hi = min(p.nz - 1, (int)floorf(fmaxf(fa, fb) + 0.01f));
+        }
+        const bool use = own && !(zlo > zhi) && s_lo <= s_hi;
+        // the lanes' slices together
+        const int first = __reduce_min_sync(0xffffffffu, use ? s_lo : p.nz);
+        const int last = __reduce_max_sync(0xffffffffu, use ? s_hi : -1);
+        if (first > last) continue;
+        // a share's slices; rows between the shares' slices at a time: len / rows_max
+        const int len = (last - first + shares) / shares;
+        const unsigned rows_max = __reduce_max_sync(0xffffffffu, __float_as_uint(use ? fabsf(g.lt * r_hd) : 0.0f));
+        const bool apart = dzs != 0.0f && (float)len > 2.1f * __uint_as_float(rows_max);
+        const int turns = apart ? v_turns : v_turns * shares, my_turn = apart ? v_turn : v_turn + v_turns * share;
+        const int s_first = first + share * len;
+        const float asn = use ? g.asn : __int_as_float(0x7fc00000);  // NaN: no slice passes the row test
+        const float inv = g.inv;
+        const size_t at = (size_t)min(s_first, last) * plane + (size_t)v * nu + min(u, nu - 1);
+        const float *pw = Gt + at, *pg = gv + at;
+        float w = __ldg(pw), gn = __ldg(pg);
+        const int col = win + (use ? c : 0);
+        for (int s = s_first; s < s_first + len; s++) {
+          const bool in = s <= last;
+          const float dz = s_z[min(s, last)] - zt, wc = in ? w : 0.0f, gc = gn;
+          if (s < last) {
+            pw += plane;
+            pg += plane;
+            w = __ldg(pw);
+            gn = __ldg(pg);
+          }
+          const float qh = __fmul_rn(fmaf(p.zr2pi, asn, dz), inv);
+          const float q = __fmul_rn(__fadd_rn(qh, 1.0f), p.hn);
+          const bool ok = fabsf(dz) <= p.z_rot && q >= 0.0f && q <= p.nrm2 && wc != 0.0f;
+          const float vv = gc * wc * q_weight_fwd(qh);  // g_vol dtheta / sum_k W_k (cuda_kernels.cuh:283) W_j
+          const float qf = floorf(q), hi = vv * (q - qf), lo = vv - hi;
+          const int at0 = col + (int)qf * W, at1 = at0 + W;
+          auto add = [&](bool mine) {
+            if (mine) {
+              const float2 d = s_win[at0], e = s_win[at1];
+              s_win[at0] = make_float2(fmaf(lo, h0, d.x), fmaf(lo, wp, d.y));
+              s_win[at1] = make_float2(fmaf(hi, h0, e.x), fmaf(hi, wp, e.y));
+            }
+            __syncwarp();
+          };
+          if (turns == 1) {
+            add(ok);
+          } else {
+            for (int k = 0; k < turns; k++) add(ok && my_turn == k);
+          }
+        }
+        __syncwarp();  // other lanes have these channels next
+      }
+    }
+  }
+  __syncthreads();
+  // channel c = its own sums + those that channel c - 1 has for it, over the windows in order
+  float* out = gD + (size_t)j * p.nr * p.nch + blockIdx.x * CH;
+  const int nc = min(CH, p.nch - (int)blockIdx.x * CH);
+  for (int e = threadIdx.x; e < nc * p.nr; e += AB_WARPS * 32) {
+    const int c = e % nc, r = e / nc;
+    float own = 0.0f, next = 0.0f;
+    for (int k = 0; k < AB_WARPS; k++) {
+      own += s_win[(size_t)k * wsize + r * W + c + 1].x;
+      next += s_win[(size_t)k * wsize + r * W + c].y;
+    }
+    out[(size_t)r * p.nch + c] = own + next;
+  }
+}
+
+// Gather without a table: a CTA owns one view and AD_CH - 1 channels; thread c
+// walks the voxels of its channel (as above), recomputes sum_k W_k of
+// every (voxel, slice) from the forward's expressions in the forward's order,
+// and adds the row contributions to two accumulators of its own in shared
+// memory, for channel c and for channel c + 1. At the end channel c = own(c) +
+// next(c - 1), in that order; the CTA's first thread only supplies
+// next(c0 - 1) for its neighbour.
 __global__ void __launch_bounds__(AD_CH, 8)
-k_bp_adjoint(const float* __restrict__ gvol, const float* __restrict__ G, float* __restrict__ gD,
-             const float2* __restrict__ view_sc, const float* __restrict__ view_z, const float* __restrict__ zslices,
-             BPParams p, float z0, float dzs, int nzp) {
+k_bp_adjoint_sums(const float* __restrict__ gvol, float* __restrict__ gD, const float2* __restrict__ view_sc,
+                  const float* __restrict__ view_z, const float* __restrict__ zslices, BPParams p, float z0,
+                  float dzs) {
   extern __shared__ float2 acc2[];  // [nr][AD_CH]: (own channel, next channel) of thread cl
-  // views of one half-turn angle run in consecutive blocks, so that they
-  // share its slice of the scale table in L2: block row b < K P/2 is view
-  // t + k P/2 with t = b / K, k = b % K; the views the forward never reads
-  // (j >= K P/2) follow in order
-  const int b = blockIdx.y, used = p.K * p.P2;
-  const int j = b < used ? (b / p.K) + (b % p.K) * p.P2 : b;
+  const int j = blockIdx.y;
   const int cl = threadIdx.x;
   const int c = blockIdx.x * (AD_CH - 1) - 1 + cl;  // channels c0 - 1 .. c0 + AD_CH - 2
   for (int r = 0; r < p.nr; r++) acc2[r * AD_CH + cl] = make_float2(0.0f, 0.0f);
@@ -206,79 +388,40 @@ k_bp_adjoint(const float* __restrict__ gvol, const float* __restrict__ G, float*
           s_lo = max(0, (int)floorf(fa) - 1);
           s_hi = min(p.nz - 1, (int)ceilf(fb) + 1);
         }
-        if constexpr (TABLE) {
-          // the voxel's weights and gradients are contiguous runs over the
-          // slices (both [.][y][x][nzp]): aligned float4 blocks, the next
-          // block's loads issued before this block's arithmetic
-          const float4* wrow = reinterpret_cast<const float4*>(G + (((size_t)t * p.ny + iy) * p.nx + ix) * nzp);
-          const float4* grow = reinterpret_cast<const float4*>(gvol + ((size_t)iy * p.nx + ix) * nzp);
-          const int e4 = s_hi >> 2;
-          int b4 = s_lo >> 2;
-          float4 wn = __ldg(wrow + b4), gn = __ldg(grow + b4);
-          for (; b4 <= e4; b4++) {
-            const float wa[4] = {wn.x, wn.y, wn.z, wn.w}, ga[4] = {gn.x, gn.y, gn.z, gn.w};
-            if (b4 < e4) {
-              wn = __ldg(wrow + b4 + 1);
-              gn = __ldg(grow + b4 + 1);
+        for (int s = s_lo; s <= s_hi; s++) {
+          const float z = __ldg(zslices + s);
+          float q_idx;
+          const float Wj = view_weight(p, g, z, &q_idx);
+          if (Wj == 0.0f) continue;
+          const float gv = __ldg(gvol + ((size_t)s * p.ny + iy) * p.nx + ix);
+          if (gv == 0.0f) continue;
+          // sum of the weights of all half turns, in the forward's order
+          float aw = 0.0f;
+          for (int k = 0; k < p.K; k++) {
+            const int jj = t + k * p.P2;
+            if (jj == j) {
+              aw += Wj;
+              continue;
             }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-              const int s = 4 * b4 + u;
-              if (s < s_lo || s > s_hi || wa[u] == 0.0f) continue;
-              float q_idx;
-              const float Wj = view_weight(p, g, __ldg(zslices + s), &q_idx);
-              if (Wj == 0.0f) continue;
-              const float scaled = ga[u] * wa[u];  // g_vol * dtheta / sum_k W_k (cuda_kernels.cuh:283)
-            const float sw = scaled * Wj;
-            const float c0v = sw * h0, c1v = sw * wp;
-            const float qf = floorf(q_idx), wq = q_idx - qf;
-            const int r = min(max((int)qf, 0), p.nr - 2);
-            float2* a0 = acc2 + r * AD_CH + cl;
-            float2 v0 = a0[0], v1 = a0[AD_CH];
-            v0.x += c0v * (1.0f - wq);
-            v0.y += c1v * (1.0f - wq);
-            v1.x += c0v * wq;
-            v1.y += c1v * wq;
-            a0[0] = v0;
-            a0[AD_CH] = v1;
-            }
+            const float ztk = __ldg(view_z + jj);
+            if (!(fabsf(z - ztk) <= p.z_rot)) continue;
+            const ViewGeo gk = view_geo(p, x, y, __ldg(view_sc + jj), ztk);
+            float qk;
+            aw += view_weight(p, gk, z, &qk);
           }
-        } else {
-          for (int s = s_lo; s <= s_hi; s++) {
-            const float z = __ldg(zslices + s);
-            float q_idx;
-            const float Wj = view_weight(p, g, z, &q_idx);
-            if (Wj == 0.0f) continue;
-            const float gv = __ldg(gvol + ((size_t)s * p.ny + iy) * p.nx + ix);
-            if (gv == 0.0f) continue;
-            // sum of the weights of all half turns, in the forward's order
-            float aw = 0.0f;
-            for (int k = 0; k < p.K; k++) {
-              const int jj = t + k * p.P2;
-              if (jj == j) {
-                aw += Wj;
-                continue;
-              }
-              const float ztk = __ldg(view_z + jj);
-              if (!(fabsf(z - ztk) <= p.z_rot)) continue;
-              const ViewGeo gk = view_geo(p, x, y, __ldg(view_sc + jj), ztk);
-              float qk;
-              aw += view_weight(p, gk, z, &qk);
-            }
-            const float scaled = gv * (p.dtheta * (1.0f / aw));  // cuda_kernels.cuh:283
-            const float sw = scaled * Wj;
-            const float c0v = sw * h0, c1v = sw * wp;
-            const float qf = floorf(q_idx), wq = q_idx - qf;
-            const int r = min(max((int)qf, 0), p.nr - 2);
-            float2* a0 = acc2 + r * AD_CH + cl;
-            float2 v0 = a0[0], v1 = a0[AD_CH];
-            v0.x += c0v * (1.0f - wq);
-            v0.y += c1v * (1.0f - wq);
-            v1.x += c0v * wq;
-            v1.y += c1v * wq;
-            a0[0] = v0;
-            a0[AD_CH] = v1;
-          }
+          const float scaled = gv * (p.dtheta * (1.0f / aw));  // cuda_kernels.cuh:283
+          const float sw = scaled * Wj;
+          const float c0v = sw * h0, c1v = sw * wp;
+          const float qf = floorf(q_idx), wq = q_idx - qf;
+          const int r = min(max((int)qf, 0), p.nr - 2);
+          float2* a0 = acc2 + r * AD_CH + cl;
+          float2 v0 = a0[0], v1 = a0[AD_CH];
+          v0.x += c0v * (1.0f - wq);
+          v0.y += c1v * (1.0f - wq);
+          v1.x += c0v * wq;
+          v1.y += c1v * wq;
+          a0[0] = v0;
+          a0[AD_CH] = v1;
         }
       }
     }
@@ -290,13 +433,17 @@ k_bp_adjoint(const float* __restrict__ gvol, const float* __restrict__ G, float*
   }
 }
 
-// gvt[vox][s] = gvol[s][vox] (s < nz), 0 for the padding up to nzp.
-__global__ void k_adj_gvol_t(const float* __restrict__ gvol, float* __restrict__ gvt, int nxy, int nz, int nzp) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)nxy * nzp) return;
-  const long vox = i / nzp;
-  const int sl = (int)(i % nzp);
-  gvt[i] = sl < nz ? __ldg(gvol + (size_t)sl * nxy + vox) : 0.0f;
+// out[s][x][y] = in[s][y][x], 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256)
+k_transpose_slices(const float* __restrict__ in, float* __restrict__ out, int nx, int ny) {
+  __shared__ float tile[32][33];
+  const size_t slice = (size_t)blockIdx.z * nx * ny;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  for (int i = ty; i < 32; i += 8)
+    if (x0 + tx < nx && y0 + i < ny) tile[i][tx] = __ldg(in + slice + (size_t)(y0 + i) * nx + x0 + tx);
+  __syncthreads();
+  for (int i = ty; i < 32; i += 8)
+    if (x0 + i < nx && y0 + tx < ny) out[slice + (size_t)(x0 + i) * ny + y0 + tx] = tile[tx][i];
 }
 
 // ---------------------------------------------------------------------------
@@ -512,34 +659,71 @@ k_taps_reduce(const float* __restrict__ partial, int nblk, int ntaps, float* __r
 
 }  // namespace
 
+namespace {
+// Channels of a CTA: the windows of all its warps together at most 60 KB, so
+// that three CTAs share an SM (up to 64 rows; taller detectors take 12
+// channels and fewer CTAs).
+int band_channels(int nr) { return std::max(12, std::min(63, 60 * 1024 / (AB_WARPS * 8 * nr) - 1)); }
+
+size_t band_smem(int nr, int nz) {
+  return sizeof(float2) * (size_t)AB_WARPS * (band_channels(nr) + 1) * nr + sizeof(float) * (size_t)nz;
+}
+
+size_t scale_smem(int nv_max) {
+  return (size_t)nv_max * (AN_WARPS * 32 * sizeof(float2) + sizeof(float)) + 32 * sizeof(float);
+}
+}  // namespace
+
+bool bp_adjoint_table_ok(const BPParams& p, int nv_max) {
+  return band_smem(p.nr, p.nz) <= 200 * 1024 && scale_smem(nv_max) <= 200 * 1024;
+}
+
 cudaError_t launch_bp_adjoint(const float* gvol, float* gD, const float2* sc, const float* vz, const float* zs,
-                              const BPParams& p, float z0, float dzs, float* scale_table, bool fill_table,
-                              float* gvol_t, cudaStream_t s) {
-  if (scale_table && fill_table) {
-    dim3 g((unsigned)((p.nx + AN_TX - 1) / AN_TX), (unsigned)((p.ny + AN_TY - 1) / AN_TY),
-           (unsigned)((p.nz + AN_ZS - 1) / AN_ZS));
-    k_bp_adjoint_scale<<<g, AN_TX * AN_TY, 0, s>>>(scale_table, sc, vz, zs, p, bp_adjoint_nzp(p.nz));
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+                              const BPParams& p, float z0, float dzs, float* scale_table, int table_angles,
+                              bool fill_table, float* gvol_t, float reach, int nv_max, cudaStream_t s) {
+  cudaError_t e;
+  if (!scale_table) {
+    dim3 grid((unsigned)((p.nch + AD_CH - 2) / (AD_CH - 1)), (unsigned)p.V);
+    const size_t smem = (size_t)p.nr * AD_CH * sizeof(float2);
+    if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(k_bp_adjoint_sums, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      (int)smem)) != cudaSuccess)
+      return e;
+    k_bp_adjoint_sums<<<grid, AD_CH, smem, s>>>(gvol, gD, sc, vz, zs, p, z0, dzs);
+    return cudaGetLastError();
   }
-  dim3 grid((unsigned)((p.nch + AD_CH - 2) / (AD_CH - 1)), (unsigned)p.V);
-  const size_t smem = (size_t)p.nr * AD_CH * sizeof(float2);
-  auto kern = scale_table ? k_bp_adjoint<true> : k_bp_adjoint<false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  if (scale_table) {
-    // the gradient volume with the table's layout [y][x][nzp]
-    const int nzp = bp_adjoint_nzp(p.nz);
-    const long n = (long)p.nx * p.ny * nzp;
-    k_adj_gvol_t<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gvol, gvol_t, p.nx * p.ny, p.nz, nzp);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    gvol = gvol_t;
-  }
-  kern<<<grid, AD_CH, smem, s>>>(gvol, scale_table, gD, sc, vz, zs, p, z0, dzs, bp_adjoint_nzp(p.nz));
-  return cudaGetLastError();
+  // the gradient volume with the voxels of a column next to each other, for the angles whose inner axis is y
+  const dim3 tg((unsigned)((p.nx + 31) / 32), (unsigned)((p.ny + 31) / 32), (unsigned)p.nz);
+  k_transpose_slices<<<tg, 256, 0, s>>>(gvol, gvol_t, p.nx, p.ny);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  // the views the forward never reads
+  const int used = p.K * p.P2;
+  const size_t view = (size_t)p.nr * p.nch;
+  if (used < p.V && (e = cudaMemsetAsync(gD + used * view, 0, sizeof(float) * view * (p.V - used), s)) != cudaSuccess)
+    return e;
+  const size_t an_smem = scale_smem(nv_max), ab_smem = band_smem(p.nr, p.nz);
+  if ((e = cudaFuncSetAttribute(k_bp_adjoint_scale, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)an_smem)) !=
+          cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_bp_adjoint_band, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ab_smem)) !=
+          cudaSuccess)
+    return e;
+  const int ch = band_channels(p.nr);
+  // one group of the table's angles after another, in launches that a grid's y takes
+  const int most = std::max(1, 65535 / std::max(p.K, 1));
+  for (int g0 = 0; g0 < p.P2; g0 += table_angles)
+    for (int t0 = g0; t0 < std::min(p.P2, g0 + table_angles); t0 += most) {
+      const int nt = std::min(most, std::min(p.P2, g0 + table_angles) - t0);
+      float* G = scale_table + (size_t)(t0 - g0) * p.nz * p.nx * p.ny;
+      if (fill_table) {
+        const dim3 g((unsigned)(((long)p.nx * p.ny + AN_WARPS * 32 - 1) / (AN_WARPS * 32)), (unsigned)nt,
+                     (unsigned)((p.nz + 31) / 32));
+        k_bp_adjoint_scale<<<g, AN_WARPS * 32, an_smem, s>>>(G, sc, vz, zs, p, t0, reach, nv_max);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      }
+      const dim3 g((unsigned)((p.nch + ch - 1) / ch), (unsigned)(nt * p.K));
+      k_bp_adjoint_band<<<g, AB_WARPS * 32, ab_smem, s>>>(gvol, gvol_t, G, gD, sc, vz, zs, p, z0, dzs, t0, reach, ch);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+  return cudaSuccess;
 }
 
 cudaError_t launch_thicken_adjoint(const float* gvol, float* gvn, const int* off, const int* ridx, const float* w,

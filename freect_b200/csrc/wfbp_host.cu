@@ -1177,30 +1177,43 @@ WFBP_API int wfbp_backproject_adjoint(wfbp_ctx* ctx, const float* g_native, floa
   float dzs = ctx->nz > 1 ? (ctx->z_native[ctx->nz - 1] - ctx->z_native[0]) / (float)(ctx->nz - 1) : 0.0f;
   for (int i = 0; i < ctx->nz && dzs != 0.0f; i++)
     if (fabsf(ctx->z_native[i] - (z0 + (float)i * dzs)) > 1e-3f * fabsf(dzs)) dzs = 0.0f;
-  // the per-(voxel, theta~) scale table when it is small enough (a few GB);
-  // otherwise the gather recomputes the weight sums
-  const size_t n = (size_t)ctx->P2 * bp_adjoint_nzp(ctx->nz) * ctx->nx * ctx->ny;
-  const bool want_table = ctx->ext.adjoint_scale_table == 0 && n * sizeof(float) <= kAdjointTableBytes;
-  if (want_table && n > ctx->adj_scale_n) {
+  // The per-(voxel, theta~) scale table: whole when it fits in 6 GB (kept until
+  // the views or slices change), else for as many half-turn angles as fit at a
+  // time, refilled in every call. A refilled table costs a weight sum per
+  // (voxel, angle, slice) and a pass over it, the gather without a table a sum
+  // per (voxel, view, slice) with all its views' geometry (64 rows, 256 x 256 x
+  // 64: 10 against 270 ms), so that form is left to memory too small for one
+  // angle's weights.
+  const size_t per_angle = (size_t)ctx->nz * ctx->nx * ctx->ny;
+  int angles = (int)std::min<size_t>(ctx->P2, kAdjointTableBytes / sizeof(float) / per_angle);
+  if (angles > 0 && angles < ctx->P2) {
+    const int groups = (ctx->P2 + angles - 1) / angles;  // equal groups
+    angles = (ctx->P2 + groups - 1) / groups;
+  }
+  const size_t n = per_angle * angles;
+  const bool want_table =
+      ctx->ext.adjoint_scale_table == 0 && angles > 0 && bp_adjoint_table_ok(p, ctx->bp_nv_max);
+  if (want_table && (n > ctx->adj_scale_n || per_angle > ctx->adj_gvt_n)) {
     free_dev(ctx->d_adj_scale);
     free_dev(ctx->d_adj_gvt);
     ctx->adj_scale_valid = false;
-    const size_t ngt = (size_t)bp_adjoint_nzp(ctx->nz) * ctx->nx * ctx->ny;
     if (cudaMalloc(&ctx->d_adj_scale, n * sizeof(float)) == cudaSuccess &&
-        cudaMalloc(&ctx->d_adj_gvt, ngt * sizeof(float)) == cudaSuccess) {
+        cudaMalloc(&ctx->d_adj_gvt, per_angle * sizeof(float)) == cudaSuccess) {
       ctx->adj_scale_n = n;
+      ctx->adj_gvt_n = per_angle;
     } else {
       cudaGetLastError();  // too large for the free memory: recompute the sums instead
       free_dev(ctx->d_adj_scale);
       free_dev(ctx->d_adj_gvt);
-      ctx->adj_scale_n = 0;
+      ctx->adj_scale_n = ctx->adj_gvt_n = 0;
     }
   }
-  float* table = want_table && ctx->d_adj_scale && ctx->d_adj_gvt && n <= ctx->adj_scale_n ? ctx->d_adj_scale
-                                                                                              : nullptr;
+  float* table = want_table && ctx->d_adj_scale && ctx->d_adj_gvt ? ctx->d_adj_scale : nullptr;
+  const bool whole = angles == ctx->P2;
   CUDA_TRY(ctx, launch_bp_adjoint(g_native, g_filtered, ctx->d_view_sc, ctx->d_view_z, ctx->d_z_native, p, z0, dzs,
-                                  table, table && !ctx->adj_scale_valid, ctx->d_adj_gvt, (cudaStream_t)stream));
-  if (table) ctx->adj_scale_valid = true;
+                                  table, angles, table && !(whole && ctx->adj_scale_valid), ctx->d_adj_gvt,
+                                  ctx->bp_reach, ctx->bp_nv_max, (cudaStream_t)stream));
+  if (table) ctx->adj_scale_valid = whole;
   return WFBP_OK;
 }
 

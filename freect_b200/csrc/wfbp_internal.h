@@ -172,7 +172,8 @@ struct wfbp_ctx {
   size_t tg_partial_n = 0;
   float* d_adj_scale = nullptr;     // backprojection adjoint: per-(voxel, theta~) weight dtheta / sum_k W_k
   size_t adj_scale_n = 0;
-  float* d_adj_gvt = nullptr;       // backprojection adjoint: gradient as [ny][nx][nzp]
+  float* d_adj_gvt = nullptr;       // backprojection adjoint: gradient as [nz][nx][ny]
+  size_t adj_gvt_n = 0;
   bool adj_scale_valid = false;     // the table matches the current views and slices
 
   // mixed precision: Toeplitz operand planes for the tensor-core filter
@@ -306,14 +307,16 @@ int tc_choose_bn(int nch);
 // requested slices list[0..nzr) (list == nullptr: 0..nzr-1)
 cudaError_t launch_thicken(const float* vn, float* out, const int* off, const int* idx, const float* w,
                            const float* ws, int nxy, int nzr, cudaStream_t s, const int* list = nullptr);
-// slice stride of the backprojection adjoint's scale table [P/2][ny][nx][nzp]
-inline int bp_adjoint_nzp(int nz) { return (nz + 3) / 4 * 4; }
-// scale_table: [P/2][ny][nx][nzp] weights dtheta / sum_k W_k, filled first
-// when fill_table is set; nullptr: the gather recomputes the weight sums.
-// gvol_t: [ny][nx][nzp] scratch for the transposed gradient (table path).
+// scale_table: [table_angles][nz][nx ny] weights dtheta / sum_k W_k, filled
+// first when fill_table is set (for table_angles half-turn angles at a time;
+// fewer than P/2: refilled for each group of angles); nullptr: the gather
+// recomputes the weight sums. gvol_t: [nz][nx][ny] scratch for the transposed
+// gradient (table path). reach, nv_max: slices' view reach and the most views
+// of one angle reaching a 32-slice slab (bp_reach).
 cudaError_t launch_bp_adjoint(const float* gvol, float* gD, const float2* sc, const float* vz, const float* zs,
-                              const BPParams& p, float z0, float dzs, float* scale_table, bool fill_table,
-                              float* gvol_t, cudaStream_t s);
+                              const BPParams& p, float z0, float dzs, float* scale_table, int table_angles,
+                              bool fill_table, float* gvol_t, float reach, int nv_max, cudaStream_t s);
+bool bp_adjoint_table_ok(const BPParams& p, int nv_max);  // the table kernels take this geometry
 cudaError_t launch_thicken_adjoint(const float* gvol, float* gvn, const int* off, const int* ridx, const float* w,
                                    int nxy, int nz, cudaStream_t s);
 cudaError_t launch_rebin_adj_cols(const float* bidx, int nch, int q8, int* cnt, int* cidx, float* cw, int maxl,

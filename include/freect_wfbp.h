@@ -206,7 +206,8 @@ typedef struct wfbp_ext {
   int filtered_layout;        /* wfbp_layout of the stage API (default REFERENCE) */
   int adjoint_scale_table;    /* 0: the backprojection adjoint keeps a per-(voxel, half-turn angle)
                                  weight table dtheta / sum_k W_k when it fits in 6 GB, computed on
-                                 the first adjoint call after the views or slices change;
+                                 the first adjoint call after the views or slices change; a larger
+                                 one is computed in every call, as many angles at a time as fit;
                                  -1: never (the adjoint recomputes the weight sums) */
   int reserved[5];
 } wfbp_ext;
