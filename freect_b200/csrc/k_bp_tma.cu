@@ -74,6 +74,28 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// Clusters: barrier over all threads of the cluster's CTAs (release / acquire,
+// which orders their shared-memory accesses), this CTA's rank, a word of
+// another CTA's shared memory.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t saddr, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared(uint32_t saddr, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(saddr), "f"(v) : "memory");
+}
+
 // Geometry of a pair of columns for one view, stored so that 16-byte
 // shared-memory loads give both columns' fields as float2 operands of the
 // packed FP32x2 instructions (FFMA2 / FADD2 / FMUL2). GeoP carries the row
@@ -182,8 +204,12 @@ __device__ __forceinline__ void bp_fused_zero(const ThickFuse& tf, int bz, int w
 // One column tile (bt.tx x bt.ty columns, SL slices from slab bz) of one scan.
 // `ring` counts the theta~ steps this CTA has run through its two-stage
 // ring before this tile (stage = ring & 1, phase = (ring >> 1) & 1), so a
-// persistent CTA continues the barriers' phases from tile to tile. Returns
-// the number of ring steps the tile used: p.P2, or 0 for a tile entirely
+// persistent CTA continues the barriers' phases from tile to tile. The tile
+// sums the half-turn angles [tb, te). With bt.nc > 1 the CTA is one of a
+// cluster of bt.nc that share the tile's angles: the CTAs leave their sums in
+// shared memory, and CTA r adds them in chunk order for its warps w = r mod nc
+// and writes those columns. RAW writes the plain sums (a batch's chunk).
+// Returns the number of ring steps the tile used: te - tb, or 0 for a tile entirely
 // outside the reconstruction FOV (whose voxels are written as 0, the value
 // the reference leaves there). A bounded wait that gave up sets the failure
 // word (the CTA must stop).
@@ -193,7 +219,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
                                         const float* __restrict__ zslices,
                                         const BPParams& p, const BPTile& bt, int bx, int by, int bz,
                                         unsigned long long* __restrict__ count, int* __restrict__ err, uint8_t* smem,
-                                        uint32_t ring, const ThickFuse& tf) {
+                                        uint32_t ring, const ThickFuse& tf, int tb, int te, bool raw) {
   constexpr bool HALF = !std::is_same<T, float>::value;
   using Geo = typename std::conditional<ZC, GeoP, GeoQ>::type;
   constexpr int NPW = CPW / 2;  // column pairs per warp
@@ -240,6 +266,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
     const float ya = ycoord(iy0), yb = ycoord(min(iy0 + bt.ty - 1, p.ny - 1));
     const float xn = fminf(fmaxf(0.0f, xa), xb), yn = fminf(fmaxf(0.0f, ya), yb);
     if (xn * xn + yn * yn > p.fov_half2 * 1.0001f + 1e-3f) {
+      if (tb > 0 && !raw) return 0;  // a cluster's first CTA writes
       if (warp < NW && my_s < p.nz) {
         const size_t plane = (size_t)p.nx * p.ny;
         for (int c = 0; c < CPG; c++) {
@@ -265,8 +292,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
     const unsigned below = (1u << lane) - 1u;
     int issued_upto = 0;
     bool failed = false;
-    for (int t = 0; t < p.P2; t++) {
-      const uint32_t g = ring + (uint32_t)t;
+    for (int t = tb; t < te; t++) {
+      const uint32_t g = ring + (uint32_t)(t - tb);
       const int s = (int)(g & 1u);
       const uint32_t u = g >> 1;
       int ok = 1;
@@ -275,7 +302,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         failed = true;
         break;
       }
-      if (FUSE && tf.out && t == min(1, p.P2 - 1)) {
+      if (FUSE && tf.out && t == min(tb + 1, te - 1)) {
         // the slab's fused-thickening records, copied while the consumers work
         // on the first stage and published by this stage's full-barrier arrive
         const int2 fr = tf.slab_tab[bz];
@@ -347,7 +374,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         const int2 vi = vinfo[s * bt.nv_max + v];
         tma_load_3d(slots + ((size_t)s * bt.nv_max + v) * bt.slot_bytes, map, &full[s], 0, vi.y, vi.x);
       }
-      issued_upto = t + 1;
+      issued_upto = t - tb + 1;
     }
     if (failed && lane == 0) {
       *s_fail = 1;
@@ -358,7 +385,13 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         mbar_wait(&full[g & 1u], (g >> 1) & 1u);
       }
     }
-    return p.P2;
+    __syncwarp();
+    if (FUSE && bt.nc > 1) {  // the consumers' barriers below
+      __syncthreads();
+      cluster_sync();
+      cluster_sync();
+    }
+    return te - tb;
   }
 
   // ---------------- consumers ----------------
@@ -386,8 +419,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   const float hrow = 0.5f * p.nrm2;  // rows [0, nr - 2] as centre and half width (records without the cull)
   const float2 mhrow2 = make_float2(-hrow, -hrow);
 
-  for (int t = 0; t < p.P2; t++) {
-    const uint32_t g = ring + (uint32_t)t;
+  for (int t = tb; t < te; t++) {
+    const uint32_t g = ring + (uint32_t)(t - tb);
     const int s = (int)(g & 1u);
     const uint32_t u = g >> 1;
     if (!mbar_wait(&full[s], u & 1u)) {
@@ -549,14 +582,37 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
     if (lane == 0) mbar_arrive(&empty[s]);
   }
 
+  bool mine = true;  // this CTA writes this warp's columns
+  if (FUSE && bt.nc > 1) {
+    // the chunks' sums of this warp's columns, added in chunk order
+    const uint32_t part = smem_u32(smem + L.part) + (uint32_t)((warp * CPG * 32 + lane) * 4);
+    const uint32_t rank = cluster_rank();
+    __syncthreads();  // the ring is idle in this CTA
+#pragma unroll
+    for (int c = 0; c < CPG; c++) st_shared(part + c * 128, (c & 1) ? vacc[c / 2].y : vacc[c / 2].x);
+    cluster_sync();
+    mine = warp % bt.nc == (int)rank;
+    if (mine) {
+#pragma unroll
+      for (int c = 0; c < CPG; c++) {
+        float v = ld_cluster(part + c * 128, 0);
+        for (int r = 1; r < bt.nc; r++) v += ld_cluster(part + c * 128, (uint32_t)r);
+        if (c & 1) vacc[c / 2].y = v;
+        else vacc[c / 2].x = v;
+      }
+    }
+    cluster_sync();  // no CTA ends, or reuses its shared memory, while another reads it
+  }
+
   // write the slab: columns outside the grid or the FOV keep the 0 the
   // reference leaves there
   const unsigned my_cols = (active_mask >> (grp * CPG)) & ((1u << CPG) - 1u);
   float vals[CPG];
+  const float scale = raw ? 1.0f : p.dtheta;
 #pragma unroll
   for (int c = 0; c < CPG; c++)
-    vals[c] = ((my_cols >> c) & 1u) ? p.dtheta * ((c & 1) ? vacc[c / 2].y : vacc[c / 2].x) : 0.0f;
-  if (my_s < p.nz) {
+    vals[c] = ((my_cols >> c) & 1u) ? scale * ((c & 1) ? vacc[c / 2].y : vacc[c / 2].x) : 0.0f;
+  if (mine && my_s < p.nz) {
     const size_t plane = (size_t)p.nx * p.ny;
 #pragma unroll
     for (int c = 0; c < CPG; c++) {
@@ -565,7 +621,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       if (ix < p.nx && iy < p.ny) vol[(size_t)my_s * plane + (size_t)iy * p.nx + ix] = vals[c];
     }
   }
-  if (FUSE && tf.out)
+  if (FUSE && tf.out && mine)
     bp_fused_thicken<CPW, SL, CPG>(tf, vals, reinterpret_cast<const int*>(smem + L.fuse),
                                    reinterpret_cast<volatile int*>(nvs)[10], warp, lane, ix0, iy0, bt, p);
   if (COUNT) {
@@ -573,7 +629,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0 && cnt) atomicAdd(count, cnt);
   }
-  return p.P2;
+  return te - tb;
 }
 
 // CTAs per SM the launch bounds of the one-tile kernel ask for: three 9-warp
@@ -587,7 +643,8 @@ constexpr int bp_min_ctas() {
   return NW > 8 ? 1 : (BATCH ? (CU == 4 && SL == 16) : (CU == 4 || SL == 16)) ? 3 : 2;
 }
 
-// One tile per CTA: grid (tiles x, tiles y, SL-slice slabs).
+// One tile per CTA: grid (tiles x, tiles y, SL-slice slabs x chunks of angles);
+// the chunks of a tile are a cluster along z.
 template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT>
 __global__ void __launch_bounds__((NW + 1) * 32, bp_min_ctas<NW, CU, SL>())
 k_bp_tma(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, const float2* __restrict__ view_sc,
@@ -597,13 +654,15 @@ k_bp_tma(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, const
   // it starts at the (128-byte aligned) base of the CTA's window
   extern __shared__ __align__(128) uint8_t smem[];
   bp_init_barriers(smem, NW);
+  const int chunk = (int)blockIdx.z % bt.nc;
   bp_tile<T, CPW, CU, NW, SL, ZC, COUNT, true>(&map, vol, view_sc, view_z, zslices, p, bt, blockIdx.x, blockIdx.y,
-                                 bt.zb0 + blockIdx.z, count, err, smem, 0u, tf);
+                                 bt.zb0 + (int)blockIdx.z / bt.nc, count, err, smem, 0u, tf,
+                                 bp_chunk_begin(chunk, bt.nc, p.P2), bp_chunk_begin(chunk + 1, bt.nc, p.P2), false);
 }
 
 // Persistent launch over the column tiles of several scans: each CTA takes
-// the next work item (scan, tile x, tile y, slab) from a global counter until
-// the list is exhausted. Items are listed by decreasing estimated cost.
+// the next work item (scan | chunk of angles << 24, tile x, tile y, slab) from
+// a global counter until the list is exhausted. Items are listed by decreasing estimated cost.
 template <typename T, int CPW, int CU, int NW, int SL, bool ZC>
 __global__ void __launch_bounds__((NW + 1) * 32, bp_min_ctas<NW, CU, SL, true>())
 k_bp_tma_batch(const BpScan* __restrict__ scans, const int4* __restrict__ items, int n_items,
@@ -618,12 +677,14 @@ k_bp_tma_batch(const BpScan* __restrict__ scans, const int4* __restrict__ items,
     const int it = words[9];
     if (it >= n_items || words[8] != 0) break;
     const int4 w = items[it];
-    const BpScan* sd = scans + w.x;
+    const BpScan* sd = scans + (w.x & 0xffffff);
+    const int chunk = w.x >> 24, nc = sd->nc;
     const BPParams p = sd->p;
     const BPTile bt = sd->bt;
-    ring += (uint32_t)bp_tile<T, CPW, CU, NW, SL, ZC, false, false>(&sd->map, sd->vol, sd->view_sc, sd->view_z,
-                                                 sd->zslices, p, bt, w.y, w.z, w.w, nullptr, err, smem, ring,
-                                                 sd->tf);
+    float* vol = sd->vol + (size_t)chunk * p.nz * p.ny * p.nx;
+    ring += (uint32_t)bp_tile<T, CPW, CU, NW, SL, ZC, false, false>(
+        &sd->map, vol, sd->view_sc, sd->view_z, sd->zslices, p, bt, w.y, w.z, w.w, nullptr, err, smem, ring, sd->tf,
+        bp_chunk_begin(chunk, nc, p.P2), bp_chunk_begin(chunk + 1, nc, p.P2), nc > 1);
     __syncthreads();  // the tile's shared memory and words[9] are free again
   }
 }
@@ -645,23 +706,26 @@ cudaError_t launch_one(const CUtensorMap& map, float* vol, const float2* sc,
                        const float* vz, const float* zs, const BPParams& p, const BPTile& bt,
                        unsigned long long* count, int* err, cudaStream_t s, const ThickFuse& tf) {
   const int nslab = (p.nz + SL - 1) / SL;
+  if (bt.nc < 1 || bt.nc > BP_MAX_CHUNKS) return cudaErrorInvalidValue;
   if (bt.zb0 < 0 || bt.zb0 >= nslab || bt.nzb < 0 || bt.zb0 + bt.nzb > nslab) return cudaErrorInvalidValue;
   dim3 grid((unsigned)((p.nx + bt.tx - 1) / bt.tx), (unsigned)((p.ny + bt.ty - 1) / bt.ty),
-            (unsigned)(bt.nzb ? bt.nzb : nslab - bt.zb0));
-  constexpr int threads = (NW + 1) * 32;
-  cudaError_t e;
-  if (count) {
-    e = prepare_kernel<NW>(k_bp_tma<T, CPW, CU, NW, SL, ZC, true>, bt.smem_bytes);
-    if (e != cudaSuccess) return e;
-    k_bp_tma<T, CPW, CU, NW, SL, ZC, true><<<grid, threads, bt.smem_bytes, s>>>(map, vol, sc, vz, zs, p, bt, count,
-                                                                             err, tf);
-  } else {
-    e = prepare_kernel<NW>(k_bp_tma<T, CPW, CU, NW, SL, ZC, false>, bt.smem_bytes);
-    if (e != cudaSuccess) return e;
-    k_bp_tma<T, CPW, CU, NW, SL, ZC, false><<<grid, threads, bt.smem_bytes, s>>>(map, vol, sc, vz, zs, p, bt, count,
-                                                                              err, tf);
-  }
-  return cudaGetLastError();
+            (unsigned)((bt.nzb ? bt.nzb : nslab - bt.zb0) * bt.nc));
+  auto kern = count ? k_bp_tma<T, CPW, CU, NW, SL, ZC, true> : k_bp_tma<T, CPW, CU, NW, SL, ZC, false>;
+  cudaError_t e = prepare_kernel<NW>(kern, bt.smem_bytes);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((NW + 1) * 32);
+  cfg.dynamicSmemBytes = (size_t)bt.smem_bytes;
+  cfg.stream = s;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
+  cluster.val.clusterDim.z = (unsigned)bt.nc;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = bt.nc > 1 ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kern, map, vol, sc, vz, zs, p, bt, count, err, tf);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <typename T, int CPW, int CU, int NW, int SL>
@@ -702,7 +766,20 @@ cudaError_t launch_elem(const CUtensorMap& map, float* vol, const float2* sc,
   return cudaErrorInvalidValue;
 }
 
+__global__ void k_sum_chunks(const float* __restrict__ part, float* __restrict__ vol, float scale, int nc, size_t n) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    float v = __ldg(part + i);
+    for (int c = 1; c < nc; c++) v += __ldg(part + (size_t)c * n + i);
+    vol[i] = scale * v;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_sum_chunks(const float* part, float* vol, float scale, int nc, size_t n, cudaStream_t s) {
+  k_sum_chunks<<<(unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, s>>>(part, vol, scale, nc, n);
+  return cudaGetLastError();
+}
 
 // Shared-memory bytes of one launch configuration.
 size_t bp_tma_smem_bytes(const BPTile& bt, int elem_bytes) {

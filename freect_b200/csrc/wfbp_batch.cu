@@ -25,6 +25,7 @@ struct wfbp_batch {
   std::vector<wfbp_ctx*> ctx;
   std::vector<void*> reb, filt;
   std::vector<float*> scales, native;
+  std::vector<float*> part;         // chunk sums [nc][nz][ny][nx] of scans with several chunks of angles, else null
   wfbp_bp_config cfg{};
   std::vector<BPTile> tiles;
   BpScan* d_scans = nullptr;
@@ -138,8 +139,9 @@ int build_plan(wfbp_batch* b) {
                                                 std::to_string(b->cfg.tile_y) + "/" +
                                                 std::to_string(b->cfg.cols_per_step) + " does not fit scan " +
                                                 std::to_string(i));
-    if (bt.zc != b->zc) {
+    if (bt.zc != b->zc || bt.nc > 1) {  // chunks of angles are work items here, no cluster
       bt.zc = b->zc;
+      bt.nc = 1;
       bt.smem_bytes = (int)bp_tma_smem_bytes(bt, 4);
       if (bt.smem_bytes > 220 * 1024)
         return bfail(b, WFBP_ERR_UNSUPPORTED, "backprojection configuration does not fit scan " + std::to_string(i));
@@ -155,7 +157,8 @@ int build_plan(wfbp_batch* b) {
     // FP16 row pairs hold the rows divided by the scan's pair_scale (a power
     // of two): the write-back's 2 pi / P takes it back, exactly
     if (b->precision == WFBP_PRECISION_MIXED) hs[i].p.dtheta *= c->pair_scale;
-    hs[i].vol = b->native[i];
+    hs[i].nc = c->bp_nc;
+    hs[i].vol = c->bp_nc > 1 ? b->part[i] : b->native[i];
     hs[i].view_sc = c->d_view_sc;
     hs[i].view_z = c->d_view_z;
     hs[i].zslices = c->d_z_native;
@@ -176,7 +179,8 @@ int build_plan(wfbp_batch* b) {
             if (x * x + y * y <= r2) cols++;
           }
         for (int sl = 0; sl < (int)nv.size(); sl++)
-          items.push_back({make_int4(i, bx, by, sl), (double)cols * nv[sl] + 1.0});
+          for (int ch = 0; ch < c->bp_nc; ch++)
+            items.push_back({make_int4(i | ch << 24, bx, by, sl), ((double)cols * nv[sl] + 1.0) / c->bp_nc});
       }
   }
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& c) { return a.cost > c.cost; });
@@ -196,6 +200,19 @@ int build_plan(wfbp_batch* b) {
   return WFBP_OK;
 }
 
+// Scan i's requested slices from its native volume, or from its chunk sums.
+int thicken_scan(wfbp_batch* b, int i, float* volume, cudaStream_t s) {
+  wfbp_ctx* c = b->ctx[i];
+  if (c->bp_nc > 1) {
+    const float scale = wfbp_detail::backprojection_params(c).dtheta *
+                        (b->precision == WFBP_PRECISION_MIXED ? c->pair_scale : 1.0f);
+    const cudaError_t e = launch_sum_chunks(b->part[i], b->native[i], scale, c->bp_nc, (size_t)c->nz * c->ny * c->nx, s);
+    if (e != cudaSuccess)
+      return wfbp_detail::set_error(c, WFBP_ERR_CUDA, std::string("chunk sums: ") + cudaGetErrorString(e));
+  }
+  return wfbp_thicken(c, b->native[i], volume, s);
+}
+
 }  // namespace
 
 WFBP_API int wfbp_batch_destroy(wfbp_batch* b) {
@@ -208,6 +225,7 @@ WFBP_API int wfbp_batch_destroy(wfbp_batch* b) {
     for (void* p : b->filt) cudaFree(p);
     for (float* p : b->scales) cudaFree(p);
     for (float* p : b->native) cudaFree(p);
+    for (float* p : b->part) cudaFree(p);
     cudaFree(b->d_next);
     cudaFree(b->d_err);
     for (float* p : b->raw_d) cudaFree(p);
@@ -248,6 +266,9 @@ WFBP_API int wfbp_batch_create(wfbp_ctx* const* ctxs, int n, wfbp_batch** out) {
     if (!e) e = cudaMalloc(&f, filt);
     if (!e && scal) e = cudaMalloc(&s, scal);
     if (!e) e = cudaMalloc(&v, nat);
+    void* pt = nullptr;
+    if (!e && b->ctx[i]->bp_nc > 1) e = cudaMalloc(&pt, nat * b->ctx[i]->bp_nc);
+    b->part.push_back(static_cast<float*>(pt));
     b->reb.push_back(r);
     b->filt.push_back(f);
     b->scales.push_back(static_cast<float*>(s));
@@ -257,18 +278,34 @@ WFBP_API int wfbp_batch_create(wfbp_ctx* const* ctxs, int n, wfbp_batch** out) {
   if (cudaMalloc(&b->d_next, sizeof(unsigned)) || cudaMalloc(&b->d_err, sizeof(int)) ||
       cudaMemset(b->d_err, 0, sizeof(int)) || cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking))
     return bad(WFBP_ERR_CUDA);
-  // default configuration: the first candidate every scan fits
+  // Default configuration, the reasons of a context's (default_bp_tile): 8 x 16
+  // columns / 8 warps / 16 slices where two such CTAs fit an SM for every scan
+  // (the persistent kernel's registers allow no third), else 16 x 20 / 20 / 16,
+  // else the first candidate every scan fits.
+  auto fits = [&](const wfbp_bp_config& c, int ctas) {
+    for (int i = 0; i < n; i++) {
+      BPTile bt;
+      if ((b->ctx[i]->ext.bp_slab && b->ctx[i]->ext.bp_slab != c.slab) ||
+          !wfbp_detail::size_backprojection(b->ctx[i], c.tile_x, c.tile_y, c.cols_per_step, c.consumer_warps, c.slab,
+                                            &bt) ||
+          ctas * (bt.smem_bytes + 1024) > 228 * 1024)
+        return false;
+    }
+    return true;
+  };
   int st = WFBP_ERR_UNSUPPORTED;
+  const wfbp_bp_config narrow = {8, 16, 8, 8, 16}, wide = {16, 20, 8, 20, 16};
+  if (fits(narrow, 2)) {
+    b->cfg = narrow;
+    st = build_plan(b);
+  } else if (fits(wide, 1)) {
+    b->cfg = wide;
+    st = build_plan(b);
+  }
   for (int k = 0; k < wfbp_detail::n_bp_candidates() && st; k++) {
     wfbp_detail::bp_candidate(k, &b->cfg.tile_x, &b->cfg.tile_y, &b->cfg.cols_per_step, &b->cfg.consumer_warps,
                               &b->cfg.slab);
-    bool fits = true;
-    for (int i = 0; i < n && fits; i++) {
-      BPTile bt;
-      fits = wfbp_detail::size_backprojection(b->ctx[i], b->cfg.tile_x, b->cfg.tile_y, b->cfg.cols_per_step,
-                                              b->cfg.consumer_warps, b->cfg.slab, &bt);
-    }
-    if (fits) st = build_plan(b);
+    if (fits(b->cfg, 1)) st = build_plan(b);
   }
   if (st) return bad(st);
   *out = b;
@@ -366,7 +403,7 @@ WFBP_API int wfbp_batch_run(wfbp_batch* b, const float* const* raws, float* cons
                                        b->d_scans, b->d_items, b->n_items, b->d_next, b->d_err, b->smem, b->grid, s);
     }
     for (int i = 0; i < n && !st && !e; i++) {
-      st = wfbp_thicken(b->ctx[i], b->native[i], volumes[i], s);
+      st = thicken_scan(b, i, volumes[i], s);
       if (st) b->err = "scan " + std::to_string(i) + ": " + wfbp_last_error(b->ctx[i]);
     }
     cudaGraph_t graph = nullptr;
@@ -455,10 +492,10 @@ WFBP_API int wfbp_batch_run_host(wfbp_batch* b, const float* const* raws_host, f
     std::vector<int4> split;
     split.reserve(b->h_items.size());
     for (const int4& w : b->h_items)
-      if (w.x < k) split.push_back(w);  // stable: each group keeps the cost order
+      if ((w.x & 0xffffff) < k) split.push_back(w);  // stable: each group keeps the cost order
     const int na = (int)split.size();
     for (const int4& w : b->h_items)
-      if (w.x >= k) split.push_back(w);
+      if ((w.x & 0xffffff) >= k) split.push_back(w);
     cudaFree(b->d_items_split);
     b->d_items_split = nullptr;
     BCUDA(b, cudaMalloc(&b->d_items_split, sizeof(int4) * std::max<size_t>(split.size(), 1)));
@@ -504,7 +541,7 @@ WFBP_API int wfbp_batch_run_host(wfbp_batch* b, const float* const* raws_host, f
                                             b->d_next, b->d_err, b->smem, b->grid, s));
     }
     for (int i = i0; i < i1; i++) {
-      int st = wfbp_thicken(b->ctx[i], b->native[i], b->vol_d[i], s);
+      int st = thicken_scan(b, i, b->vol_d[i], s);
       if (st) return bfail(b, st, "scan " + std::to_string(i) + ": " + wfbp_last_error(b->ctx[i]));
     }
     return WFBP_OK;

@@ -311,6 +311,11 @@ void bp_reach(wfbp_ctx* ctx, const std::vector<float>& table) {
     }
   }
   ctx->bp_reach = (float)reach;
+  // the channel window of the default shape's 8 x 16 columns (size_bp_tile)
+  const double vx = ctx->rp.recon_fov / ctx->nx, vy = ctx->rp.recon_fov / ctx->ny;
+  const double window = ceil(hypot(7 * vx, 15 * vy) * ctx->gp.pixel_scale) + 5.0;
+  ctx->bp_nc = bp_theta_chunks(ctx->nx, ctx->ny, ctx->nz_config, ctx->P2,
+                               (size_t)std::min(window, 1.0e6) * ((ctx->nr + 3) / 4 * 4) * 4);
   ctx->bp_nv_max = std::max(1, nv_max);
   // A sample with its row in [0, nr - 2] has |z - z_j| <= cone; below z_rot
   // by a margin for rounding, the cull of cuda_kernels.cuh:232 never removes
@@ -330,9 +335,10 @@ bool size_bp_tile(const wfbp_ctx* ctx, int tx, int ty, int cu, int nw, int slab,
   b.zb0 = 0;
   b.nzb = 0;
   b.zc = ctx->bp_zcull;
+  b.nc = ctx->bp_nc;
   const double ext = sqrt(pow((b.tx - 1) * vx, 2) + pow((b.ty - 1) * vy, 2));
+  if (ext * ctx->gp.pixel_scale > 250.0) return false;  // a TMA box holds at most 256 channels
   b.W = (int)ceil(ext * ctx->gp.pixel_scale) + 5;
-  b.W = std::max(4, std::min(b.W, 256));
   b.nrp = (ctx->nr + 3) / 4 * 4;
   b.nv_max = ctx->bp_nv_max;
   b.slot_bytes = (int)((b.W * b.nrp * 4 + 127) / 128 * 128);
@@ -357,8 +363,29 @@ const int kBpCandidates[][5] = {
 // ext.bp_slab, when set, admits only configurations with slabs of that height
 bool slab_allowed(const wfbp_ctx* ctx, int slab) { return ctx->ext.bp_slab == 0 || ctx->ext.bp_slab == slab; }
 
+// The launch shape a context starts with (an autotuner may set another). The
+// kernel is bound by instruction issue and hides its latencies with resident
+// warps, and a 16-slice slab keeps more lanes inside a view's cone than a
+// 32-slice one, so: 8 x 16 columns / 8 warps / 16 slices where three CTAs fit an
+// SM (24 consumer warps), else 16 x 20 / 20 / 16 (20 warps in one CTA: wide view
+// windows, as a flying focal spot's), else the first candidate that fits.
+// Measured, ms, 16x16/4w16s32 (the first candidate) -> this rule: 16 rows 256 x
+// 256 x 26 FP32 7.93 -> 5.44; 20 rows 333 x 287 x 74 mixed 24.3 -> 17.9; 64 rows
+// 512 x 512 x 480 FP32 217.5 -> 200.5, mixed 206.9 -> 200.6; flying focal spot
+// 512 x 512 x 166 FP32 48.0 -> 46.6, where 8x16/8w8s16 (two CTAs) takes 68.1.
+bool default_bp_tile(const wfbp_ctx* ctx, BPTile* out) {
+  BPTile b;
+  if (!slab_allowed(ctx, 16)) return false;
+  if (size_bp_tile(ctx, 8, 16, 8, 8, 16, &b) && 3 * (b.smem_bytes + 1024) <= 228 * 1024) {
+    *out = b;
+    return true;
+  }
+  return size_bp_tile(ctx, 16, 20, 8, 20, 16, out);
+}
+
 bool choose_bp_tile(wfbp_ctx* ctx, const std::vector<float>& table) {
   bp_reach(ctx, table);
+  if (default_bp_tile(ctx, &ctx->bpt)) return true;
   for (auto& c : kBpCandidates) {
     if (!slab_allowed(ctx, c[4])) continue;
     BPTile b;
@@ -651,6 +678,7 @@ WFBP_API int wfbp_ctx_create(const CTGeometry* cg, const ReconConfig* rp, const 
 
   int st = slice_lists(cg, rp, ctx->z_native, ctx->z_req);
   if (st) { delete ctx; return st; }
+  ctx->nz_config = (int)ctx->z_native.size();
 
   ctx->taps.resize(ctx->nch);
   st = make_taps(cg, e.filter_window, e.filter_c, e.filter_a, e.user_taps, e.n_user_taps, ctx->taps.data(), ctx->nch);

@@ -51,7 +51,32 @@ struct BPTile {
   int slab;          // native slices per slab (32, or 16 with two column groups per warp)
   int zb0, nzb;      // slabs [zb0, zb0 + nzb) of this launch (nzb 0: all)
   int zc;            // 1: geometry records carry the table-position cull's row range (it can bind)
+  int nc;            // chunks of half-turn angles, one CTA of a cluster each (bp_theta_chunks; 1: no cluster)
 };
+
+// The half-turn angles of a voxel are summed in `bp_theta_chunks` chunks whose
+// sums are then added in order, by a cluster of as many CTAs per column tile
+// (in the persistent batch by as many work items): a small volume has too few
+// tiles to fill the chip. nz is the slice count of the context's ReconConfig
+// and the window that of the default shape, so that every launch shape, slab,
+// shard and batch of a scan sums in the same order. Split until the default
+// shape's CTAs fill one wave (444 resident, 148 where a view's channel window
+// is wide), or two where a chunk keeps 64 angles or more to spread its
+// pipeline's start over. Backprojection ms in 1 / 2 / 4 / 8 chunks: 48 x 48 x
+// 13, 209 angles .643 / .338 / .179 / .143; 147 x 132 x 21, 497 angles 3.53 /
+// 2.92 / 2.62 / 2.63; 88 x 88 x 74, 63 angles .326 / .287 / .269 / .301; 256 x
+// 256 x 26, 580 angles 5.49 / 5.43 / 5.70 / 5.88; 125 x 99 x 178, 35 angles
+// .412 / .430 / .484 / .661.
+constexpr int BP_MAX_CHUNKS = 8;
+inline int bp_theta_chunks(int nx, int ny, int nz, int P2, size_t window_bytes) {
+  const long tiles = ((long)(nx + 7) / 8) * ((ny + 15) / 16) * ((nz + 15) / 16);  // the default shape's
+  // three views in two stages, three CTAs to an SM
+  const long wave = 6 * window_bytes + 12 * 1024 <= 75 * 1024 ? 444 : 148;
+  int nc = 1;
+  while (nc < BP_MAX_CHUNKS && P2 >= 8 * nc && tiles * nc < (P2 >= 128 * nc ? 2 * wave : wave)) nc *= 2;
+  return nc;
+}
+__host__ __device__ inline int bp_chunk_begin(int chunk, int nc, int P2) { return (int)((long)P2 * chunk / nc); }
 
 // Bits of the device-side error word besides WFBP_ERR_TIMEOUT (which a
 // bounded wait that gave up stores whole): conditions the host's sizing rules
@@ -69,7 +94,7 @@ constexpr int BT_FUSE_WORDS = 384;  // shared-memory words for one slab's fused-
 constexpr int BP_GEO_BYTES_ZCULL = 48;  // column-pair record with the row range of the table-position cull
 constexpr int BP_GEO_BYTES = 32;        // column-pair record when that cull never binds
 struct BpSmem {
-  unsigned slots, vinfo, vgeo, geo, fuse, total;
+  unsigned slots, vinfo, vgeo, geo, fuse, part, total;
 };
 // Per staged view, the geometry the consumers' record pass reads (copied by
 // the producer lane that selects the view): sin and cos of the tube angle and
@@ -93,6 +118,16 @@ __host__ __device__ inline BpSmem bp_smem_layout(const BPTile& bt, int cpw) {
   o += (unsigned)(bt.nw * bt.nv_max * (cpw / 2) * (bt.zc ? BP_GEO_BYTES_ZCULL : BP_GEO_BYTES));  // column-pair records
   L.fuse = o;
   o += (unsigned)(BT_FUSE_WORDS * 4);  // the slab's fused-thickening records (ThickFuse)
+  // a cluster's chunk sums [warp][column][lane]: over the ring when they fit there (it is idle by then)
+  L.part = L.slots;
+  if (bt.nc > 1) {
+    const unsigned bytes = (unsigned)(bt.tx * bt.ty * bt.slab) * 4u;
+    if (bytes > L.vinfo - L.slots) {
+      o = (o + 15u) & ~15u;
+      L.part = o;
+      o += bytes;
+    }
+  }
   L.total = o;
   return L;
 }
@@ -129,6 +164,7 @@ struct wfbp_ctx {
   int n_readings = 0, raw_rows = 0, raw_ch = 0;
   int reading_offset = 0;           // first reading's index within the whole scan
   std::vector<float> z_native, z_req;
+  int nz_config = 0;                // native slices of the ReconConfig (wfbp_set_slices does not change it)
   std::vector<float> view_table;    // table position of each view (host copy)
   std::vector<float> taps;          // symmetric half taps h[0..nch-1]
   std::vector<int> thick_off;       // CSR over requested slices
@@ -195,6 +231,7 @@ struct wfbp_ctx {
   bool bp_tma_ok = false;
   BPTile bpt;
   float bp_reach = 0.0f;            // slab-level view prefilter half width (mm)
+  int bp_nc = 1;                    // chunks of half-turn angles (bp_theta_chunks)
   int bp_nv_max = 1;                // most views of one theta~ reaching a slab
   int bp_zcull = 1;                 // 0: the table-position cull (|z - z_j| > z_rot) never removes a
                                     // sample whose row lies in [0, nr - 2] (cone shorter than z_rot)
@@ -292,7 +329,10 @@ struct alignas(64) BpScan {
   const float* view_z;
   const float* zslices;
   ThickFuse tf;                 // fused thickening (tf.out == nullptr: none)
+  int nc;                       // chunks of half-turn angles; > 1: vol is [nc][nz][ny][nx] chunk sums
 };
+// native volume = scale * (chunk sums added in order), the batch's scans of more than one chunk
+cudaError_t launch_sum_chunks(const float* part, float* vol, float scale, int nc, size_t n, cudaStream_t s);
 cudaError_t bp_tma_encode_map(const void* D, int elem_half2, const BPParams& p, const BPTile& bt, CUtensorMap* map);
 cudaError_t launch_backproject_tma_batch(int elem_half2, int cpw, int cu, int nw, int slab, int zc, const BpScan* scans,
                                          const int4* items, int n_items, unsigned* next, int* err, int smem_bytes,
