@@ -157,14 +157,16 @@ __device__ __forceinline__ int fft_word(int k1, int t) {
   return k1 * BLK + (t ^ chunk_xor<R3>(R2 > 1 ? t / R3 : k1));
 }
 
-// Rows 2 i, 2 i + 1 of X [M][nch] -> Y, rows as they are or (TR) in the
-// backprojection layout Y[view][channel][nrp] (row m = view nr + row). A CTA
-// holds G transforms at a time and walks pairs of rows with the grid's stride:
-// the twiddles of pass 1 stay in its threads' registers.
+// Rows of X [V][nr][nch] -> Y, rows as they are or (TR) in the backprojection
+// layout Y[view][channel][nrp]. Rows 2 i and 2 i + 1 of a view are a pair (an
+// odd view's last row is alone), so that a row's roundings do not depend on
+// where a range of views begins. A CTA holds G transforms at a time and walks
+// the pairs with the grid's stride: the twiddles of pass 1 stay in its
+// threads' registers.
 template <int N, bool TR>
 __global__ void __launch_bounds__(N / 16 > FF_THREADS ? N / 16 : FF_THREADS, N / 16 > FF_THREADS ? 2 : 4)
 k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __restrict__ taps,
-             const float2* __restrict__ spec, const float2* __restrict__ tw, long M, int nch, int nr, int nrp) {
+             const float2* __restrict__ spec, const float2* __restrict__ tw, int V, int nch, int nr, int nrp) {
   constexpr int R2 = FftShape<N>::R2, R3 = FftShape<N>::R3, T = N / 16;
   constexpr int CTA = T > FF_THREADS ? T : FF_THREADS, G = CTA / T;
   constexpr int PAD = R2 > 1 ? R3 : 0, BLK = T + PAD, PLANE = 16 * BLK + (R2 > 1 ? 0 : 16);
@@ -184,11 +186,15 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
   for (int k = 1; k < 16; k++) tw1[k] = __ldg(tw + t * k);
   __syncthreads();
 
-  const long pairs = (M + 1) / 2, steps = (pairs + G - 1) / G;
+  const unsigned per_view = (unsigned)(nr + 1) / 2;
+  const long pairs = (long)V * per_view, steps = (pairs + G - 1) / G;
   int buf = 0;
   for (long st = blockIdx.x; st < steps; st += gridDim.x, buf ^= 1) {
-    const long pair = st * G + g, m = 2 * pair;
-    const bool has_a = m < M, has_b = m + 1 < M;
+    const long pair = st * G + g;
+    const long v = pairs < (1l << 31) ? (long)((unsigned)pair / per_view) : pair / per_view;
+    const int r0 = 2 * (int)(pair - v * per_view);
+    const long m = v * nr + r0;  // row of X
+    const bool has_a = pair < pairs, has_b = has_a && r0 + 1 < nr;
     // ---- pass 1: points n = n1 T + t, n1 < 8 (the others are padding), and
     // their left neighbours (from L1)
     float2 a[8], l[8];
@@ -372,25 +378,12 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
       }
     }
     if constexpr (TR) {
-      const long v0 = M < (1l << 31) ? (long)((unsigned)m / (unsigned)nr) : m / nr;
-      const int r0 = (int)(m - v0 * nr);
-      const bool wrap = r0 + 1 == nr;  // the pair straddles two views
-      const long v1 = wrap ? v0 + 1 : v0;
-      const int r1 = wrap ? 0 : r0 + 1;
-      if (!wrap && has_b && r0 % 2 == 0) {
-        float* y = Y + (size_t)v0 * nch * nrp + r0;
+      float* y = Y + (size_t)v * nch * nrp + r0;  // nrp is a multiple of 4, r0 even
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int n = j * T + t;
-          if (n < nch) *reinterpret_cast<float2*>(y + (size_t)n * nrp) = a[j];
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int n = j * T + t;
-          if (n < nch && has_a) Y[((size_t)v0 * nch + n) * nrp + r0] = a[j].x;
-          if (n < nch && has_b) Y[((size_t)v1 * nch + n) * nrp + r1] = a[j].y;
-        }
+      for (int j = 0; j < 8; j++) {
+        const int n = j * T + t;
+        if (n < nch && has_b) *reinterpret_cast<float2*>(y + (size_t)n * nrp) = a[j];
+        else if (n < nch && has_a) y[(size_t)n * nrp] = a[j].x;
       }
     } else {
 #pragma unroll
@@ -445,7 +438,7 @@ k_filter_spectrum(const float* __restrict__ taps, int nch, int N, int R2, int R3
 }
 
 template <int N, bool TR>
-cudaError_t launch_n(const float* x, float* y, const float* taps, const float2* spec, const float2* tw, long rows,
+cudaError_t launch_n(const float* x, float* y, const float* taps, const float2* spec, const float2* tw, int V,
                      int nch, int nr, int nrp, cudaStream_t s) {
   constexpr int R2 = FftShape<N>::R2, R3 = FftShape<N>::R3, T = N / 16;
   constexpr int CTA = T > FF_THREADS ? T : FF_THREADS, G = CTA / T;
@@ -458,21 +451,21 @@ cudaError_t launch_n(const float* x, float* y, const float* taps, const float2* 
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CTA, smem)) != cudaSuccess) return e;
-  const long steps = ((rows + 1) / 2 + G - 1) / G;
+  const long steps = ((long)V * ((nr + 1) / 2) + G - 1) / G;
   const unsigned grid = (unsigned)std::max(1L, std::min<long>(steps, (long)sms * std::max(per_sm, 1)));
-  kern<<<grid, CTA, smem, s>>>(x, y, taps, spec, tw, rows, nch, nr, nrp);
+  kern<<<grid, CTA, smem, s>>>(x, y, taps, spec, tw, V, nch, nr, nrp);
   return cudaGetLastError();
 }
 
 template <bool TR>
 cudaError_t launch_by_size(const float* x, float* y, const float* taps, const float2* spec, const float2* tw, int N,
-                           long rows, int nch, int nr, int nrp, cudaStream_t s) {
+                           int V, int nch, int nr, int nrp, cudaStream_t s) {
   switch (N) {
-    case 256: return launch_n<256, TR>(x, y, taps, spec, tw, rows, nch, nr, nrp, s);
-    case 512: return launch_n<512, TR>(x, y, taps, spec, tw, rows, nch, nr, nrp, s);
-    case 1024: return launch_n<1024, TR>(x, y, taps, spec, tw, rows, nch, nr, nrp, s);
-    case 2048: return launch_n<2048, TR>(x, y, taps, spec, tw, rows, nch, nr, nrp, s);
-    case 4096: return launch_n<4096, TR>(x, y, taps, spec, tw, rows, nch, nr, nrp, s);
+    case 256: return launch_n<256, TR>(x, y, taps, spec, tw, V, nch, nr, nrp, s);
+    case 512: return launch_n<512, TR>(x, y, taps, spec, tw, V, nch, nr, nrp, s);
+    case 1024: return launch_n<1024, TR>(x, y, taps, spec, tw, V, nch, nr, nrp, s);
+    case 2048: return launch_n<2048, TR>(x, y, taps, spec, tw, V, nch, nr, nrp, s);
+    case 4096: return launch_n<4096, TR>(x, y, taps, spec, tw, V, nch, nr, nrp, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -505,8 +498,8 @@ cudaError_t launch_filter_spectrum(const float* d_taps, int nch, int N, float2* 
 }
 
 cudaError_t launch_filter_fft(const float* x, float* y, const float* d_taps, const float2* spec, const float2* tw, int N,
-                              long rows, int nch, int nr, int nrp, bool transposed, cudaStream_t s) {
-  if (nch >= N / 2 || rows < 1) return cudaErrorInvalidValue;
-  return transposed ? launch_by_size<true>(x, y, d_taps, spec, tw, N, rows, nch, nr, nrp, s)
-                    : launch_by_size<false>(x, y, d_taps, spec, tw, N, rows, nch, nr, nrp, s);
+                              int V, int nch, int nr, int nrp, bool transposed, cudaStream_t s) {
+  if (nch >= N / 2 || V < 1) return cudaErrorInvalidValue;
+  return transposed ? launch_by_size<true>(x, y, d_taps, spec, tw, N, V, nch, nr, nrp, s)
+                    : launch_by_size<false>(x, y, d_taps, spec, tw, N, V, nch, nr, nrp, s);
 }

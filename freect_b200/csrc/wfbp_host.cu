@@ -1047,8 +1047,8 @@ int filter_rows_f32(wfbp_ctx* ctx, const float* x, float* y, long rows, bool bpl
                     cudaStream_t s) {
   if (ctx->fft_n && fft) {
     if (spectrum) CUDA_TRY(ctx, launch_filter_spectrum(ctx->d_taps, ctx->nch, ctx->fft_n, ctx->d_fft_spec, s));
-    CUDA_TRY(ctx, launch_filter_fft(x, y, ctx->d_taps, ctx->d_fft_spec, ctx->d_fft_tw, ctx->fft_n, rows, ctx->nch,
-                                    ctx->nr, ctx->bpt.nrp, bpl, s));
+    CUDA_TRY(ctx, launch_filter_fft(x, y, ctx->d_taps, ctx->d_fft_spec, ctx->d_fft_tw, ctx->fft_n,
+                                    (int)(rows / ctx->nr), ctx->nch, ctx->nr, ctx->bpt.nrp, bpl, s));
   } else if (bpl) {
     CUDA_TRY(ctx, launch_filter_f32_tr(x, y, ctx->d_taps, rows, ctx->nch, ctx->nr, ctx->bpt.nrp, s));
   } else {

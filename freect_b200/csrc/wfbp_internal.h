@@ -300,7 +300,7 @@ int filter_fft_size(int nch);
 void filter_fft_twiddles(int N, float2* tw);
 cudaError_t launch_filter_spectrum(const float* d_taps, int nch, int N, float2* spec, cudaStream_t s);
 cudaError_t launch_filter_fft(const float* x, float* y, const float* d_taps, const float2* spec, const float2* tw, int N,
-                              long rows, int nch, int nr, int nrp, bool transposed, cudaStream_t s);
+                              int V, int nch, int nr, int nrp, bool transposed, cudaStream_t s);
 // Thickening fused into the TMA backprojection's write-back: a requested
 // slice whose native slices (the thickening CSR row) all lie in one slab is
 // formed from that slab's registers and written to `out`; the other

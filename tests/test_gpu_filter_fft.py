@@ -28,6 +28,7 @@ DEV = torch.device("cuda", 0)
 
 def make_ctx(nch, nr, layout, P=8, rotations=2.5):
     spec = scans.tiny(nch=nch, nr=nr, P=P, rotations=rotations, nx=8, n_slices=1)
+    spec.fov = 8.0  # a channel window that every shape holds
     tube, table = spec.views()
     cg, _ = wfbp.configure_geometry(spec.meta(), table)
     ctx = wfbp.Context(cg, spec.recon_config(), wfbp.make_ext(filtered_layout=layout), device=0)
