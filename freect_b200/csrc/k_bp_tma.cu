@@ -116,6 +116,15 @@ struct __align__(16) GeoQ {
   int2 addr;
   float2 wp;
 };
+// Record of the reference layout's form (REFQ): k_bp's own arithmetic per
+// slice, q = (((z - zt) + zr2pi asn) inv + 1) hn with the roundings that
+// kernel has, so that a sample at the edge of the detector falls the same way.
+struct __align__(16) GeoR {
+  float2 inv, asn;  // 1 / (l_hat tan(cone)), asin(p_hat / R) (an invalid record: 1, -1e30)
+  int2 addr;
+  float2 wp;
+};
+static_assert(sizeof(GeoR) == BP_GEO_BYTES, "record sizes of bp_smem_layout");
 static_assert(sizeof(GeoP) == BP_GEO_BYTES_ZCULL && sizeof(GeoQ) == BP_GEO_BYTES, "record sizes of bp_smem_layout");
 
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
@@ -213,7 +222,7 @@ __device__ __forceinline__ void bp_fused_zero(const ThickFuse& tf, int bz, int w
 // outside the reconstruction FOV (whose voxels are written as 0, the value
 // the reference leaves there). A bounded wait that gave up sets the failure
 // word (the CTA must stop).
-template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT, bool FUSE>
+template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT, bool FUSE, bool REFQ = false>
 __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict__ vol,
                                         const float2* __restrict__ view_sc, const float* __restrict__ view_z,
                                         const float* __restrict__ zslices,
@@ -221,7 +230,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
                                         unsigned long long* __restrict__ count, int* __restrict__ err, uint8_t* smem,
                                         uint32_t ring, const ThickFuse& tf, int tb, int te, bool raw) {
   constexpr bool HALF = !std::is_same<T, float>::value;
-  using Geo = typename std::conditional<ZC, GeoP, GeoQ>::type;
+  static_assert(!REFQ || (!HALF && !ZC), "the reference layout's form: FP32 rows, its own cull test");
+  using Geo = typename std::conditional<REFQ, GeoR, typename std::conditional<ZC, GeoP, GeoQ>::type>::type;
   constexpr int NPW = CPW / 2;  // column pairs per warp
   // SL = 32: the warp's 32 lanes are 32 slices of each of its CPW columns.
   // SL = 16: lanes 0-15 and 16-31 are 16 slices of two column groups of
@@ -450,9 +460,17 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         t_hat = fmaf(gx, vf.y, gy * vf.x);
         zt = vf.z;
       }
-      const float l_hat = bp_sqrt(p.R2 - p_hat * p_hat) - t_hat;
-      const float A = p.zr2pi * bp_asin(p.rR * p_hat);
-      const float inv = bp_rcp(l_hat * p.tanc);
+      float A, inv;  // REFQ: A is the arcsine itself
+      if constexpr (REFQ) {
+        const float4 vf = *reinterpret_cast<const float4*>(&vg);
+        const float l_hat = fmaf(-gy, vf.x, fmaf(-gx, vf.y, sqrtf(fmaf(-p_hat, p_hat, p.R2))));
+        A = asinf(p.rR * p_hat);
+        inv = 1.0f / (l_hat * p.tanc);
+      } else {
+        const float l_hat = bp_sqrt(p.R2 - p_hat * p_hat) - t_hat;
+        A = p.zr2pi * bp_asin(p.rR * p_hat);
+        inv = bp_rcp(l_hat * p.tanc);
+      }
       const float p_idx = p.kp - (p_hat * p.ps + p.c0);
       const float pf = floorf(p_idx);
       // floor(p_idx) >= 0 and ceil(p_idx) <= nch - 2 (cuda_kernels.cuh:259-263)
@@ -467,7 +485,10 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       const float wp = p_idx - pf;
       float* gf = reinterpret_cast<float*>(wgeo + v * NPW + (gc >> 1)) + (gc & 1);
       constexpr int O = ZC ? 4 : 0;  // float offset of addr / wp behind the row range
-      if constexpr (ZC) {
+      if constexpr (REFQ) {
+        gf[0] = valid ? inv : 1.0f;
+        gf[2] = valid ? A : -1.0e30f;
+      } else if constexpr (ZC) {
         gf[0] = bq;
         gf[2] = cq;
         // rows q in [0, nr - 2] (cuda_kernels.cuh:259-263) of views within z_rot (:232)
@@ -505,12 +526,27 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       }
       for (int v = 0; v < nv; v++) {
         const Geo* gpv = wgeo + v * NPW + (grp * CPG + c0) / 2;
+        float dz = 0.0f;
+        bool zok = true;
+        if constexpr (REFQ) {
+          dz = zl - reinterpret_cast<const float4*>(&vgeo[s * bt.nv_max + v])->z;
+          zok = fabsf(dz) <= p.z_rot;  // cuda_kernels.cuh:232
+        }
 #pragma unroll
         for (int u2 = 0; u2 < CU / 2; u2++) {
           const Geo g = gpv[u2];
-          const float2 q = __ffma2_rn(zl2, g.bq, g.cq);
+          float2 q, qh;
           bool okx, oky;
-          if constexpr (ZC) {
+          if constexpr (REFQ) {
+            qh = __fmul2_rn(__ffma2_rn(make_float2(p.zr2pi, p.zr2pi), g.asn, make_float2(dz, dz)), g.inv);
+            q = __fmul2_rn(__fadd2_rn(qh, make_float2(1.0f, 1.0f)), make_float2(p.hn, p.hn));
+            okx = zok && q.x >= 0.0f && q.x <= p.nrm2;
+            oky = zok && q.y >= 0.0f && q.y <= p.nrm2;
+          } else {
+            q = __ffma2_rn(zl2, g.bq, g.cq);
+          }
+          if constexpr (REFQ) {
+          } else if constexpr (ZC) {
             const float2 dq = __fadd2_rn(q, neg2(g.qmid));
             okx = fabsf(dq.x) <= g.qhw.x;
             oky = fabsf(dq.y) <= g.qhw.y;
@@ -559,9 +595,10 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
           }
           const float2 gval = __ffma2_rn(wq, __fadd2_rn(bot, neg2(top)), top);
           // W(q) of cuda_kernels.cuh:79-93 with |q_hat| = |q - hn| / hn
-          const float2 a = __fadd2_rn(q, mhn2);
-          const float2 tt = __fmul2_rn(make_float2(__saturatef(fmaf(fabsf(a.x), k1, -1.5f)),
-                                                   __saturatef(fmaf(fabsf(a.y), k1, -1.5f))),
+          const float2 a = REFQ ? qh : __fadd2_rn(q, mhn2);
+          const float ka = REFQ ? 2.5f : k1;
+          const float2 tt = __fmul2_rn(make_float2(__saturatef(fmaf(fabsf(a.x), ka, -1.5f)),
+                                                   __saturatef(fmaf(fabsf(a.y), ka, -1.5f))),
                                        pi2);
           float2 W = __ffma2_rn(half2c, make_float2(__cosf(tt.x), __cosf(tt.y)), half2c);
           W.x = okx ? W.x : 0.0f;
@@ -660,6 +697,53 @@ k_bp_tma(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, const
                                  bp_chunk_begin(chunk, bt.nc, p.P2), bp_chunk_begin(chunk + 1, bt.nc, p.P2), false);
 }
 
+// The same on the reference layout's rows (transposed, rows_to_channels), with
+// k_bp's arithmetic.
+template <int CPW, int CU, int NW, int SL, bool COUNT>
+__global__ void __launch_bounds__((NW + 1) * 32, bp_min_ctas<NW, CU, SL>())
+k_bp_tma_refq(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, const float2* __restrict__ view_sc,
+              const float* __restrict__ view_z, const float* __restrict__ zslices, BPParams p, BPTile bt,
+              unsigned long long* __restrict__ count, int* __restrict__ err) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  bp_init_barriers(smem, NW);
+  const int chunk = (int)blockIdx.z % bt.nc;
+  ThickFuse none;
+  none.out = nullptr;
+  bp_tile<float, CPW, CU, NW, SL, false, COUNT, true, true>(
+      &map, vol, view_sc, view_z, zslices, p, bt, blockIdx.x, blockIdx.y, (int)blockIdx.z / bt.nc, count, err, smem, 0u,
+      none, bp_chunk_begin(chunk, bt.nc, p.P2), bp_chunk_begin(chunk + 1, bt.nc, p.P2), false);
+}
+
+// out[view][channel][row] (rows padded to nrp, the padding not written) from
+// FP32 rows in[view][row][channel], or FP16 rows times their power-of-two
+// scales [view][row] (exact). One CTA per view and 32 channels, 64 rows at a
+// time through shared memory: full lines on both sides.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_rows_to_channels(const T* __restrict__ in, const float* __restrict__ scales, float* __restrict__ out, int nr, int nch,
+                   int nrp) {
+  __shared__ float tile[64][33];
+  const size_t v = blockIdx.x;
+  const int c0 = blockIdx.y * 32, nc = min(32, nch - c0);
+  for (int r0 = 0; r0 < nr; r0 += 64) {
+    const int n = min(64, nr - r0);
+    for (int e = threadIdx.x; e < n * 32; e += 256) {
+      const int r = e / 32, c = e % 32;
+      if (c < nc) {
+        const T x = in[(v * nr + r0 + r) * nch + c0 + c];
+        if constexpr (std::is_same<T, float>::value) tile[r][c] = x;
+        else tile[r][c] = __half2float(x) * __ldg(scales + v * nr + r0 + r);
+      }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * nc; e += 256) {
+      const int c = e / n, r = e % n;
+      out[(v * nch + c0 + c) * nrp + r0 + r] = tile[r][c];
+    }
+    __syncthreads();
+  }
+}
+
 // Persistent launch over the column tiles of several scans: each CTA takes
 // the next work item (scan | chunk of angles << 24, tile x, tile y, slab) from
 // a global counter until the list is exhausted. Items are listed by decreasing estimated cost.
@@ -701,6 +785,24 @@ cudaError_t prepare_kernel(K* kern, int smem) {
   return e;
 }
 
+template <typename... Args>
+cudaError_t launch_cluster(void (*kern)(Args...), dim3 grid, int threads, int smem, int nc, cudaStream_t s,
+                           Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
+  cluster.val.clusterDim.z = (unsigned)nc;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = nc > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 template <typename T, int CPW, int CU, int NW, int SL, bool ZC>
 cudaError_t launch_one(const CUtensorMap& map, float* vol, const float2* sc,
                        const float* vz, const float* zs, const BPParams& p, const BPTile& bt,
@@ -713,19 +815,7 @@ cudaError_t launch_one(const CUtensorMap& map, float* vol, const float2* sc,
   auto kern = count ? k_bp_tma<T, CPW, CU, NW, SL, ZC, true> : k_bp_tma<T, CPW, CU, NW, SL, ZC, false>;
   cudaError_t e = prepare_kernel<NW>(kern, bt.smem_bytes);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((NW + 1) * 32);
-  cfg.dynamicSmemBytes = (size_t)bt.smem_bytes;
-  cfg.stream = s;
-  cudaLaunchAttribute cluster;
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
-  cluster.val.clusterDim.z = (unsigned)bt.nc;
-  cfg.attrs = &cluster;
-  cfg.numAttrs = bt.nc > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, map, vol, sc, vz, zs, p, bt, count, err, tf);
-  return e != cudaSuccess ? e : cudaGetLastError();
+  return launch_cluster(kern, grid, (NW + 1) * 32, bt.smem_bytes, bt.nc, s, map, vol, sc, vz, zs, p, bt, count, err, tf);
 }
 
 template <typename T, int CPW, int CU, int NW, int SL>
@@ -829,6 +919,47 @@ cudaError_t launch_backproject_tma(const void* D, int elem_half2, float row_scal
   const ThickFuse& f = tf ? *tf : none;
   if (elem_half2) return launch_elem<uint32_t>(map, vol, sc, vz, zs, p, bt, count, err, s, f);
   return launch_elem<float>(map, vol, sc, vz, zs, p, bt, count, err, s, f);
+}
+
+// The shapes of the reference layout's form: the default ones (default_bp_tile)
+// and the smallest tile.
+#define WFBP_REFQ_SHAPES(X) X(16, 8, 8, 16) X(16, 8, 20, 16) X(4, 4, 16, 32)
+
+bool bp_refq_supported(const BPTile& bt) {
+  const int cpw = bt.tx * bt.ty / bt.nw;
+#define WFBP_SUP(C, U, N, S) \
+  if (cpw == C && bt.cu == U && bt.nw == N && bt.slab == S) return true;
+  WFBP_REFQ_SHAPES(WFBP_SUP)
+#undef WFBP_SUP
+  return false;
+}
+
+cudaError_t launch_rows_to_channels(const void* rows, const float* f16_scales, float* out, int V, int nr, int nch,
+                                    int nrp, cudaStream_t s) {
+  const dim3 g((unsigned)V, (unsigned)((nch + 31) / 32));
+  if (f16_scales) k_rows_to_channels<<<g, 256, 0, s>>>((const __half*)rows, f16_scales, out, nr, nch, nrp);
+  else k_rows_to_channels<<<g, 256, 0, s>>>((const float*)rows, f16_scales, out, nr, nch, nrp);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_backproject_refq(const float* D, float* vol, const float2* sc, const float* vz, const float* zs,
+                                    const BPParams& p, const BPTile& bt, unsigned long long* count, int* err,
+                                    cudaStream_t s) {
+  CUtensorMap map;
+  cudaError_t e = bp_tma_encode_map(D, 0, p, bt, &map);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((unsigned)((p.nx + bt.tx - 1) / bt.tx), (unsigned)((p.ny + bt.ty - 1) / bt.ty),
+                  (unsigned)(((p.nz + bt.slab - 1) / bt.slab) * bt.nc));
+  const int cpw = bt.tx * bt.ty / bt.nw;
+#define WFBP_ONE(C, U, N, S)                                                                                       \
+  if (cpw == C && bt.cu == U && bt.nw == N && bt.slab == S) {                                                      \
+    auto kern = count ? k_bp_tma_refq<C, U, N, S, true> : k_bp_tma_refq<C, U, N, S, false>;                        \
+    if ((e = prepare_kernel<N>(kern, bt.smem_bytes)) != cudaSuccess) return e;                                     \
+    return launch_cluster(kern, grid, (N + 1) * 32, bt.smem_bytes, bt.nc, s, map, vol, sc, vz, zs, p, bt, count, err); \
+  }
+  WFBP_REFQ_SHAPES(WFBP_ONE)
+#undef WFBP_ONE
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_backproject_tma_batch(int elem_half2, int cpw, int cu, int nw, int slab, int zc, const BpScan* scans,

@@ -183,6 +183,8 @@ void release(wfbp_ctx* ctx) {
   free_dev(ctx->d_tg_partial);
   free_dev(ctx->d_adj_scale);
   free_dev(ctx->d_adj_gvt);
+  if (ctx->refq_pool) cudaMemPoolDestroy(ctx->refq_pool);
+  ctx->refq_pool = nullptr;
   for (auto& e : ctx->ev_copy) cudaEventDestroy(e);
   ctx->ev_copy.clear();
   if (ctx->s_copy) cudaStreamDestroy(ctx->s_copy);
@@ -383,8 +385,27 @@ bool default_bp_tile(const wfbp_ctx* ctx, BPTile* out) {
   return size_bp_tile(ctx, 16, 20, 8, 20, 16, out);
 }
 
+// The reference layout's launch: a default shape, else the smallest tile; none
+// for a scan without table feed, whose records need it (k_bp then).
+void choose_refq_tile(wfbp_ctx* ctx) {
+  BPTile b;
+  ctx->refq_ok = false;
+  if (!(ctx->gp.z_rot_over_2_pi > 0.0f)) return;
+  wfbp_ext any = ctx->ext;
+  any.bp_slab = 0;  // restricts the backprojection layout's shapes only
+  std::swap(ctx->ext, any);
+  const bool fits = default_bp_tile(ctx, &b) || size_bp_tile(ctx, 8, 8, 4, 16, 32, &b);
+  std::swap(ctx->ext, any);
+  if (!fits || !bp_refq_supported(b)) return;
+  b.zc = 0;
+  b.smem_bytes = (int)bp_tma_smem_bytes(b, 4);
+  ctx->refq = b;
+  ctx->refq_ok = true;
+}
+
 bool choose_bp_tile(wfbp_ctx* ctx, const std::vector<float>& table) {
   bp_reach(ctx, table);
+  choose_refq_tile(ctx);
   if (default_bp_tile(ctx, &ctx->bpt)) return true;
   for (auto& c : kBpCandidates) {
     if (!slab_allowed(ctx, c[4])) continue;
@@ -1099,8 +1120,53 @@ int do_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* scales
   return filter_rows_f32(ctx, x, y, (long)(ve - vb) * ctx->nr, bpl, !ctx->taps_set, vb == 0, s);
 }
 
+// The reference layout's rows transposed into the backprojection layout, in
+// memory of the context's pool in stream order (calls on several streams each
+// have their own; the pool keeps what it has until the context ends), and the
+// TMA-staged kernel on them with k_bp's arithmetic: 16 rows, 256 x 256 x 26
+// FP32 11.4 ms by k_bp's gathers from L2, 6.4 here, 0.06 of them the
+// transpose. False: not done, k_bp has to (no launch fits, no memory, or the
+// stream is being captured: a graph would own the memory).
+bool backproject_refq(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol, const BPParams& p,
+                      unsigned long long* update_count, cudaStream_t s, cudaError_t* e) {
+  *e = cudaSuccess;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!ctx->refq_ok || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  if (!ctx->refq_pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cuuint64_t keep = ~0ull;
+    if (cudaMemPoolCreate(&ctx->refq_pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(ctx->refq_pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      if (ctx->refq_pool) cudaMemPoolDestroy(ctx->refq_pool);
+      ctx->refq_pool = nullptr;
+      cudaGetLastError();
+      return false;
+    }
+  }
+  void* d = nullptr;
+  if (cudaMallocFromPoolAsync(&d, sizeof(float) * (size_t)ctx->V * ctx->nch * ctx->refq.nrp, ctx->refq_pool, s) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  *e = launch_rows_to_channels(filtered, scales, (float*)d, ctx->V, ctx->nr, ctx->nch, ctx->refq.nrp, s);
+  if (*e == cudaSuccess)
+    *e = launch_backproject_refq((const float*)d, vol, ctx->d_view_sc, ctx->d_view_z, ctx->d_z_native, p, ctx->refq,
+                                 update_count, ctx->d_err, s);
+  const cudaError_t ef = cudaFreeAsync(d, s);
+  if (*e == cudaSuccess) *e = ef;
+  return true;
+}
+
 int do_backproject(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol,
-                   unsigned long long* update_count, int layout, void* stream, const ThickFuse* tf = nullptr) {
+                   unsigned long long* update_count, int layout, void* stream, const ThickFuse* tf = nullptr,
+                   bool may_allocate = true) {
   const cudaStream_t s = (cudaStream_t)stream;
   BPParams p = bp_params(ctx);
   const bool mixed = ctx->ext.precision == WFBP_PRECISION_MIXED;
@@ -1110,6 +1176,11 @@ int do_backproject(wfbp_ctx* ctx, const void* filtered, const float* scales, flo
       return fail(ctx, WFBP_ERR_UNSUPPORTED, "wfbp_backproject: no backprojection-layout launch fits this geometry");
     CUDA_TRY(ctx, launch_backproject_tma(filtered, mixed ? 1 : 0, ctx->pair_scale, vol, ctx->d_view_sc, ctx->d_view_z,
                                          ctx->d_z_native, p, ctx->bpt, update_count, ctx->d_err, s, tf));
+    return WFBP_OK;
+  }
+  cudaError_t e;
+  if (may_allocate && backproject_refq(ctx, filtered, mixed ? scales : nullptr, vol, p, update_count, s, &e)) {
+    CUDA_TRY(ctx, e);
     return WFBP_OK;
   }
   if (mixed)
@@ -1699,7 +1770,7 @@ int filter_stage(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* sca
 }
 int backproject_stage(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol, int layout,
                       void* stream) {
-  return do_backproject(ctx, filtered, scales, vol, nullptr, layout, stream);
+  return do_backproject(ctx, filtered, scales, vol, nullptr, layout, stream, nullptr, false);
 }
 int run_layout_of(const wfbp_ctx* ctx) { return run_layout(ctx); }
 int n_bp_candidates() { return (int)(sizeof(kBpCandidates) / sizeof(kBpCandidates[0])); }

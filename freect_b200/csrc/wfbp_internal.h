@@ -236,6 +236,12 @@ struct wfbp_ctx {
   int bp_zcull = 1;                 // 0: the table-position cull (|z - z_j| > z_rot) never removes a
                                     // sample whose row lies in [0, nr - 2] (cone shorter than z_rot)
 
+  // reference layout through the TMA-staged kernel: its launch (refq_ok), and
+  // the pool its transposed rows come from, in stream order
+  bool refq_ok = false;
+  BPTile refq;
+  cudaMemPool_t refq_pool = nullptr;
+
   // context-owned scratch for wfbp_run / wfbp_run_host
   void* s_rebinned = nullptr;
   void* s_filtered = nullptr;
@@ -343,6 +349,15 @@ cudaError_t launch_backproject_tma(const void* D, int elem_half2, float row_scal
                                    const float2* sc, const float* vz, const float* zs, const BPParams& p,
                                    const BPTile& bt, unsigned long long* count, int* err, cudaStream_t s,
                                    const ThickFuse* tf = nullptr);
+// Reference layout through the TMA-staged kernel: the rows transposed into the
+// backprojection layout (FP16 rows with their scales [V][nr]), then k_bp's
+// arithmetic on them.
+bool bp_refq_supported(const BPTile& bt);
+cudaError_t launch_rows_to_channels(const void* rows, const float* f16_scales, float* out, int V, int nr, int nch,
+                                    int nrp, cudaStream_t s);
+cudaError_t launch_backproject_refq(const float* D, float* vol, const float2* sc, const float* vz, const float* zs,
+                                    const BPParams& p, const BPTile& bt, unsigned long long* count, int* err,
+                                    cudaStream_t s);
 int tc_choose_bn(int nch);
 // requested slices list[0..nzr) (list == nullptr: 0..nzr-1)
 cudaError_t launch_thicken(const float* vn, float* out, const int* off, const int* idx, const float* w,
