@@ -75,15 +75,10 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
 }
 
 // Clusters: barrier over all threads of the cluster's CTAs (release / acquire,
-// which orders their shared-memory accesses), this CTA's rank, a word of
-// another CTA's shared memory.
+// which orders their shared-memory accesses), a word of another CTA's shared
+// memory.
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
 }
 __device__ __forceinline__ float ld_cluster(uint32_t saddr, uint32_t rank) {
   uint32_t a;
@@ -127,19 +122,19 @@ struct __align__(16) GeoR {
 static_assert(sizeof(GeoR) == BP_GEO_BYTES, "record sizes of bp_smem_layout");
 static_assert(sizeof(GeoP) == BP_GEO_BYTES_ZCULL && sizeof(GeoQ) == BP_GEO_BYTES, "record sizes of bp_smem_layout");
 
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// a - b: fma(b, -1, a) rounds once, like the subtraction
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
 
 // Shared memory of a CTA: the mbarriers and small words at fixed offsets
 // (they persist across the tiles of a persistent launch), then the regions
 // of bp_smem_layout for the tile's scan.
-// int [16]: [0..1] views per stage, [8] failure flag, [9] next item, [10] fused-thickening words
+// int [16]: [0..1] views per stage, [2..3] steps per stage, [8] failure flag, [9] next item
 constexpr int BT_OFF_NVS = 64;
 
 __device__ __forceinline__ void bp_init_barriers(uint8_t* smem, int nw) {
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   if (threadIdx.x == 0) {
     reinterpret_cast<int*>(smem + BT_OFF_NVS)[8] = 0;
-    reinterpret_cast<int*>(smem + BT_OFF_NVS)[10] = 0;
     for (int s = 0; s < BT_STAGES; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&full[BT_STAGES + s], nw);
@@ -150,8 +145,7 @@ __device__ __forceinline__ void bp_init_barriers(uint8_t* smem, int nw) {
   __syncthreads();
 }
 
-// Fused thickening of one slab (ThickFuse). The producer warp has copied the
-// slab's records into shared memory (fz, nfz words) while the ring filled.
+// Fused thickening of one slab (ThickFuse) from its records (fz, nfz words).
 // For every interior requested slice r each group of SL lanes (lane = slice
 // s0 + lane % SL) gathers its native values with shuffles, in the CSR order
 // and with the same FMA chain and division as k_thicken, so the result is
@@ -168,15 +162,15 @@ __device__ __forceinline__ void bp_fused_thicken(const ThickFuse& tf, const floa
   const size_t plane = (size_t)p.nx * p.ny, vox = (size_t)iy * p.nx + ix;
   nfz = min(nfz, BT_FUSE_WORDS);
   for (int pos = 0; pos + 3 <= nfz;) {
-    const int r = fz[pos], n = fz[pos + 1];
-    const float ws = __int_as_float(fz[pos + 2]);
+    const int r = __ldg(fz + pos), n = __ldg(fz + pos + 1);
+    const float ws = __int_as_float(__ldg(fz + pos + 2));
     if (n < 0 || pos + 3 + 2 * n > nfz) break;  // malformed records (host sizing guarantees otherwise)
     float acc[CPG];
 #pragma unroll
     for (int c = 0; c < CPG; c++) acc[c] = 0.0f;
     for (int e = 0; e < n; e++) {
-      const int src = grp * SL + (fz[pos + 3 + 2 * e] & (SL - 1));
-      const float wt = __int_as_float(fz[pos + 4 + 2 * e]);
+      const int src = grp * SL + (__ldg(fz + pos + 3 + 2 * e) & (SL - 1));
+      const float wt = __int_as_float(__ldg(fz + pos + 4 + 2 * e));
 #pragma unroll
       for (int c = 0; c < CPG; c++) acc[c] = fmaf(wt, __shfl_sync(0xffffffffu, vals[c], src), acc[c]);
     }
@@ -214,21 +208,26 @@ __device__ __forceinline__ void bp_fused_zero(const ThickFuse& tf, int bz, int w
 // `ring` counts the theta~ steps this CTA has run through its two-stage
 // ring before this tile (stage = ring & 1, phase = (ring >> 1) & 1), so a
 // persistent CTA continues the barriers' phases from tile to tile. The tile
-// sums the half-turn angles [tb, te). With bt.nc > 1 the CTA is one of a
-// cluster of bt.nc that share the tile's angles: the CTAs leave their sums in
-// shared memory, and CTA r adds them in chunk order for its warps w = r mod nc
-// and writes those columns. RAW writes the plain sums (a batch's chunk).
+// sums the half-turn angles of chunk `chunk` of nc. With BP_CLUSTER the CTA is
+// number `chunk` of a cluster of nc that share the tile's angles: the CTAs
+// leave their sums in shared memory, and CTA r adds them in chunk order for its
+// warps w = r mod nc and writes those columns. BP_ITEM with nc > 1 writes the
+// plain sums (a batch's chunk).
 // Returns the number of ring steps the tile used: te - tb, or 0 for a tile entirely
 // outside the reconstruction FOV (whose voxels are written as 0, the value
 // the reference leaves there). A bounded wait that gave up sets the failure
 // word (the CTA must stop).
-template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT, bool FUSE, bool REFQ = false>
+// The angles a tile sums: all of them, a chunk as a CTA of a cluster, or a
+// chunk whose plain sums a persistent batch writes.
+enum BpRange { BP_ALL, BP_CLUSTER, BP_ITEM };
+
+template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT, bool FUSE, int RANGE, bool REFQ = false>
 __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict__ vol,
                                         const float2* __restrict__ view_sc, const float* __restrict__ view_z,
                                         const float* __restrict__ zslices,
                                         const BPParams& p, const BPTile& bt, int bx, int by, int bz,
                                         unsigned long long* __restrict__ count, int* __restrict__ err, uint8_t* smem,
-                                        uint32_t ring, const ThickFuse& tf, int tb, int te, bool raw) {
+                                        uint32_t ring, const ThickFuse& tf, int chunk, int nc) {
   constexpr bool HALF = !std::is_same<T, float>::value;
   static_assert(!REFQ || (!HALF && !ZC), "the reference layout's form: FP32 rows, its own cull test");
   using Geo = typename std::conditional<REFQ, GeoR, typename std::conditional<ZC, GeoP, GeoQ>::type>::type;
@@ -243,12 +242,17 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   uint8_t* slots = smem + L.slots;                            // [STAGES][nv_max][slot_bytes]
   int2* vinfo = reinterpret_cast<int2*>(smem + L.vinfo);      // [STAGES][nv_max] (view, first channel)
   BpViewGeo* vgeo = reinterpret_cast<BpViewGeo*>(smem + L.vgeo);  // [STAGES][nv_max] the views' angle and z
-  int* nvs = reinterpret_cast<int*>(smem + BT_OFF_NVS);       // [STAGES] views, [8] failure flag
-  Geo* geo = reinterpret_cast<Geo*>(smem + L.geo);            // [warps][nv_max][NPW]
+  float2* vwin = reinterpret_cast<float2*>(smem + L.vwin);    // [nv_max] slice range the tile can use of a view (producer)
+  uint32_t* vlist = reinterpret_cast<uint32_t*>(smem + L.list);  // [STAGES][32] the lanes' views, 4 bits each
+  int* nvs = reinterpret_cast<int*>(smem + BT_OFF_NVS);       // [STAGES] views, [2 + stage] steps, [8] failure flag
+  // [warps][nv_max + 1] views of [NG][CPG / 2] records (bp_geo_view)
+  constexpr unsigned GEO_G = bp_geo_group(CPW, SL, (int)sizeof(Geo)), GEO_V = bp_geo_view(CPW, SL, (int)sizeof(Geo));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* empty = full + BT_STAGES;
   volatile int* s_fail = nvs + 8;
 
+  const int tb = RANGE == BP_ALL ? 0 : bp_chunk_begin(chunk, nc, p.P2);
+  const int te = RANGE == BP_ALL ? p.P2 : bp_chunk_begin(chunk + 1, nc, p.P2);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int ix0 = bx * bt.tx, iy0 = by * bt.ty;
   const int s0 = bz * SL;
@@ -276,7 +280,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
     const float ya = ycoord(iy0), yb = ycoord(min(iy0 + bt.ty - 1, p.ny - 1));
     const float xn = fminf(fmaxf(0.0f, xa), xb), yn = fminf(fmaxf(0.0f, ya), yb);
     if (xn * xn + yn * yn > p.fov_half2 * 1.0001f + 1e-3f) {
-      if (tb > 0 && !raw) return 0;  // a cluster's first CTA writes
+      if (RANGE == BP_CLUSTER && chunk > 0) return 0;  // the cluster's first CTA writes
       if (warp < NW && my_s < p.nz) {
         const size_t plane = (size_t)p.nx * p.ny;
         for (int c = 0; c < CPG; c++) {
@@ -312,22 +316,13 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         failed = true;
         break;
       }
-      if (FUSE && tf.out && t == min(tb + 1, te - 1)) {
-        // the slab's fused-thickening records, copied while the consumers work
-        // on the first stage and published by this stage's full-barrier arrive
-        const int2 fr = tf.slab_tab[bz];
-        const int nw = max(0, min(fr.y - fr.x, BT_FUSE_WORDS));
-        int* fz = reinterpret_cast<int*>(smem + L.fuse);
-        for (int j = lane; j < nw; j += 32) fz[j] = __ldg(tf.tab + fr.x + j);
-        if (lane == 0) nvs[10] = nw;
-        __syncwarp();
-      }
       int nv = 0;
       for (int kb = 0; kb < p.K; kb += 32) {
         const int k = kb + lane;
         const int j = t + k * p.P2;
         bool sel = false;
         int c_lo = 0;
+        float wlo = 0.0f, whi = 0.0f;
         float4 vf = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // FP32 form: the view's sin, cos, z for the records
         if (k < p.K) {
           const float zt = __ldg(view_z + j);
@@ -345,7 +340,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
             const float lhi = sqrtf(p.R2) - fminf(fminf(t1, t2), fminf(t3, t4));
             const float amin = p.zr2pi * asinf(p.rR * pmin), amax = p.zr2pi * asinf(p.rR * pmax);
             const float eps = 1e-3f * (1.0f + fabsf(zt));
-            const float wlo = zt - amax - lhi * p.tanc - eps, whi = zt - amin + lhi * p.tanc + eps;
+            wlo = zt - amax - lhi * p.tanc - eps;
+            whi = zt - amin + lhi * p.tanc + eps;
             sel = !(whi < zmn || wlo > zmx);
             const float idx_min = p.kp - (pmax * p.ps + p.c0);  // p_idx decreases with p_hat
             c_lo = max(0, min((int)floorf(idx_min) - 1, p.nch - bt.W));
@@ -356,6 +352,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         if (sel) {
           if (pos < bt.nv_max) {
             vinfo[s * bt.nv_max + pos] = make_int2(j, c_lo);
+            vwin[pos] = make_float2(wlo, whi);
             // the view's angle and z for the consumers' record pass (the
             // mixed form's FP64 tables; the FP32 form's values of the test)
             BpViewGeo* g = vgeo + s * bt.nv_max + pos;
@@ -373,6 +370,30 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
           }
         }
         nv = min(nv + __popc(m), bt.nv_max);
+      }
+      __syncwarp();
+      {
+        // lane = slice: the views, in order, whose slice range holds it
+        uint32_t list = 0u;
+        int n = 0;
+        if (nv > 1 && bt.nv_max <= BP_LIST_VIEWS)
+          for (int v = 0; v < nv; v++) {
+            const float2 w = vwin[v];
+            if (zl >= w.x && zl <= w.y) {
+              list |= n < 8 ? (uint32_t)v << (4 * n) : 0u;
+              n++;
+            }
+          }
+        const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+        // the idle record ends a list
+        if (n < 8) list |= (uint32_t)(0x11111111u * (unsigned)bt.nv_max) << (4 * n);
+        // Steps over lists cost more each (lanes on two views' samples meet in
+        // the banks, more so with FP32 rows' eight loads per pair): every view
+        // for every lane unless they save enough.
+        const bool pays = nv > 1 && bt.nv_max <= BP_LIST_VIEWS && most <= 8 &&
+                          (HALF ? 6 * most < 5 * nv : 3 * most <= 2 * nv);
+        vlist[s * 32 + lane] = pays ? list : 0x76543210u;
+        if (lane == 0) nvs[2 + s] = pays ? most : nv;
       }
       __syncwarp();
       if (lane == 0) {
@@ -396,7 +417,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       }
     }
     __syncwarp();
-    if (FUSE && bt.nc > 1) {  // the consumers' barriers below
+    if (RANGE == BP_CLUSTER) {  // the consumers' barriers below
       __syncthreads();
       cluster_sync();
       cluster_sync();
@@ -410,7 +431,27 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   for (int c = 0; c < CPG / 2; c++) vacc[c] = make_float2(0.0f, 0.0f);
   unsigned long long cnt = 0;
   const float k1 = 2.5f / p.hn;
-  Geo* wgeo = geo + (size_t)warp * bt.nv_max * NPW;
+  uint8_t* wgeo = smem + L.geo + (size_t)warp * (bt.nv_max + 1) * GEO_V;
+  // the idle records: no lane valid, zeros to sample (those every warp writes, the same)
+  for (int e = lane; e < 2 * bt.nrp; e += 32) reinterpret_cast<float*>(smem + L.zero)[e] = 0.0f;
+  if (lane < NPW) {
+    Geo* g = reinterpret_cast<Geo*>(wgeo + bt.nv_max * GEO_V + lane / (CPG / 2) * GEO_G) + lane % (CPG / 2);
+    if constexpr (REFQ) {
+      g->inv = make_float2(1.0f, 1.0f);
+      g->asn = make_float2(-1.0e30f, -1.0e30f);
+    } else {
+      g->bq = make_float2(0.0f, 0.0f);
+      g->cq = make_float2(-1.0e30f, -1.0e30f);
+    }
+    if constexpr (ZC) {
+      g->qmid = make_float2(0.0f, 0.0f);
+      g->qhw = make_float2(-1.0f, -1.0f);
+    }
+    g->addr = make_int2((int)L.zero, (int)L.zero);
+    g->wp = make_float2(0.0f, 0.0f);
+  }
+  if (REFQ && lane == 0) reinterpret_cast<float4*>(vgeo + 2 * bt.nv_max)->z = 0.0f;
+  __syncwarp();
   constexpr int VPP = 32 / CPW;  // views per geometry pass
   const int gc = lane % CPW, gv = lane / CPW;
   const int gt = warp * CPW + gc;  // tile column handled by this lane in geometry passes
@@ -426,8 +467,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   const float2 pi2 = make_float2(3.14159265f, 3.14159265f);
   const float2 half2c = make_float2(0.5f, 0.5f);
   const unsigned nrm2u = (unsigned)(p.nr - 2);
-  const float hrow = 0.5f * p.nrm2;  // rows [0, nr - 2] as centre and half width (records without the cull)
-  const float2 mhrow2 = make_float2(-hrow, -hrow);
+  const unsigned nrm2b = __float_as_uint(p.nrm2);
 
   for (int t = tb; t < te; t++) {
     const uint32_t g = ring + (uint32_t)(t - tb);
@@ -483,7 +523,9 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       const float bq = inv * p.hn;
       const float cq = p.hn * fmaf(A - zt, inv, 1.0f);
       const float wp = p_idx - pf;
-      float* gf = reinterpret_cast<float*>(wgeo + v * NPW + (gc >> 1)) + (gc & 1);
+      float* gf = reinterpret_cast<float*>(reinterpret_cast<Geo*>(wgeo + v * GEO_V + gc / CPG * GEO_G) +
+                                           (gc % CPG >> 1)) +
+                  (gc & 1);
       constexpr int O = ZC ? 4 : 0;  // float offset of addr / wp behind the row range
       if constexpr (REFQ) {
         gf[0] = valid ? inv : 1.0f;
@@ -512,6 +554,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       }
     }
     __syncwarp();
+    const uint32_t my_list = vlist[s * 32 + lane];
+    const int steps = nvs[2 + s];
 #pragma unroll
     for (int c0 = 0; c0 < CPG; c0 += CU) {
       unsigned any = 0u;  // warp-uniform: some group has an active column in this step
@@ -524,18 +568,30 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         ag[u2] = make_float2(0.0f, 0.0f);
         aw[u2] = make_float2(0.0f, 0.0f);
       }
-      for (int v = 0; v < nv; v++) {
-        const Geo* gpv = wgeo + v * NPW + (grp * CPG + c0) / 2;
+      // Each lane takes the views whose cone can hold its slice, in order; the
+      // views left out would add zeros. With every lane taking every view that
+      // reaches the slab about half the lane slots of a 16-row scanner were
+      // outside the cone (ms, every view / lists: 16 rows mixed 5.50 / 4.64,
+      // FP32 5.45 / 4.84; 20 rows 17.8 / 15.4, 17.8 / 17.3; 64 rows 39.9 / 39.4,
+      // 39.7 / 39.5; 8 x 16 / 8 / 16 slices).
+      // (Eight views to a word; more only where every lane takes every view.)
+      uint32_t list = my_list;
+      const uint8_t* gb = wgeo + grp * GEO_G + c0 / 2 * sizeof(Geo);
+      for (int i = 0; i < steps; i++) {
+        unsigned v = list & 15u;
+        list >>= 4;
+        if (i >= 8) v = (unsigned)i;
+        const Geo* gpv = reinterpret_cast<const Geo*>(gb + v * GEO_V);
         float dz = 0.0f;
         bool zok = true;
         if constexpr (REFQ) {
-          dz = zl - reinterpret_cast<const float4*>(&vgeo[s * bt.nv_max + v])->z;
+          dz = zl - reinterpret_cast<const float4*>(&vgeo[v < (unsigned)bt.nv_max ? s * bt.nv_max + v : 2 * bt.nv_max])->z;
           zok = fabsf(dz) <= p.z_rot;  // cuda_kernels.cuh:232
         }
 #pragma unroll
         for (int u2 = 0; u2 < CU / 2; u2++) {
           const Geo g = gpv[u2];
-          float2 q, qh;
+          float2 q, qh = make_float2(0.0f, 0.0f);
           bool okx, oky;
           if constexpr (REFQ) {
             qh = __fmul2_rn(__ffma2_rn(make_float2(p.zr2pi, p.zr2pi), g.asn, make_float2(dz, dz)), g.inv);
@@ -547,13 +603,13 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
           }
           if constexpr (REFQ) {
           } else if constexpr (ZC) {
-            const float2 dq = __fadd2_rn(q, neg2(g.qmid));
+            const float2 dq = sub2(q, g.qmid);
             okx = fabsf(dq.x) <= g.qhw.x;
             oky = fabsf(dq.y) <= g.qhw.y;
           } else {
-            const float2 dq = __fadd2_rn(q, mhrow2);
-            okx = fabsf(dq.x) <= hrow;
-            oky = fabsf(dq.y) <= hrow;
+            // 0 <= q <= nr - 2 (cuda_kernels.cuh:259-263): order of the bits, negative q above all
+            okx = __float_as_uint(q.x) <= nrm2b;
+            oky = __float_as_uint(q.y) <= nrm2b;
           }
           // Row index and fraction through the FP32 pipe: for 0 <= q < 2^23,
           // q + 2^23 rounded down is 2^23 + floor(q), an integer held in the
@@ -564,7 +620,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
           const float2 fq = __fadd2_rn(tq, make_float2(-8388608.0f, -8388608.0f));
           const unsigned rx = min(__float_as_uint(tq.x) - 0x4B000000u, nrm2u);
           const unsigned ry = min(__float_as_uint(tq.y) - 0x4B000000u, nrm2u);
-          const float2 wq = __fadd2_rn(q, neg2(fq));
+          const float2 wq = sub2(q, fq);
           const uint8_t* ex = smem + g.addr.x + (rx << 2);
           const uint8_t* ey = smem + g.addr.y + (ry << 2);
           float2 top, bot;
@@ -576,8 +632,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
                                            *reinterpret_cast<const float*>(ey + nrpb));
             const float2 d11 = make_float2(*reinterpret_cast<const float*>(ex + nrpb + 4),
                                            *reinterpret_cast<const float*>(ey + nrpb + 4));
-            top = __ffma2_rn(g.wp, __fadd2_rn(d10, neg2(d00)), d00);
-            bot = __ffma2_rn(g.wp, __fadd2_rn(d11, neg2(d01)), d01);
+            top = __ffma2_rn(g.wp, sub2(d10, d00), d00);
+            bot = __ffma2_rn(g.wp, sub2(d11, d01), d01);
           } else {
             // (row r, row r+1) pairs of channels pf and pf+1, interpolated
             // across channels in half2 arithmetic
@@ -593,7 +649,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
             top = make_float2(fx.x, fy.x);
             bot = make_float2(fx.y, fy.y);
           }
-          const float2 gval = __ffma2_rn(wq, __fadd2_rn(bot, neg2(top)), top);
+          const float2 gval = __ffma2_rn(wq, sub2(bot, top), top);
           // W(q) of cuda_kernels.cuh:79-93 with |q_hat| = |q - hn| / hn
           const float2 a = REFQ ? qh : __fadd2_rn(q, mhn2);
           const float ka = REFQ ? 2.5f : k1;
@@ -620,20 +676,19 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   }
 
   bool mine = true;  // this CTA writes this warp's columns
-  if (FUSE && bt.nc > 1) {
+  if constexpr (RANGE == BP_CLUSTER) {
     // the chunks' sums of this warp's columns, added in chunk order
     const uint32_t part = smem_u32(smem + L.part) + (uint32_t)((warp * CPG * 32 + lane) * 4);
-    const uint32_t rank = cluster_rank();
     __syncthreads();  // the ring is idle in this CTA
 #pragma unroll
     for (int c = 0; c < CPG; c++) st_shared(part + c * 128, (c & 1) ? vacc[c / 2].y : vacc[c / 2].x);
     cluster_sync();
-    mine = warp % bt.nc == (int)rank;
+    mine = warp % nc == chunk;
     if (mine) {
 #pragma unroll
       for (int c = 0; c < CPG; c++) {
         float v = ld_cluster(part + c * 128, 0);
-        for (int r = 1; r < bt.nc; r++) v += ld_cluster(part + c * 128, (uint32_t)r);
+        for (int r = 1; r < nc; r++) v += ld_cluster(part + c * 128, (uint32_t)r);
         if (c & 1) vacc[c / 2].y = v;
         else vacc[c / 2].x = v;
       }
@@ -645,7 +700,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   // reference leaves there
   const unsigned my_cols = (active_mask >> (grp * CPG)) & ((1u << CPG) - 1u);
   float vals[CPG];
-  const float scale = raw ? 1.0f : p.dtheta;
+  const float scale = RANGE == BP_ITEM && nc > 1 ? 1.0f : p.dtheta;
 #pragma unroll
   for (int c = 0; c < CPG; c++)
     vals[c] = ((my_cols >> c) & 1u) ? scale * ((c & 1) ? vacc[c / 2].y : vacc[c / 2].x) : 0.0f;
@@ -658,9 +713,10 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       if (ix < p.nx && iy < p.ny) vol[(size_t)my_s * plane + (size_t)iy * p.nx + ix] = vals[c];
     }
   }
-  if (FUSE && tf.out && mine)
-    bp_fused_thicken<CPW, SL, CPG>(tf, vals, reinterpret_cast<const int*>(smem + L.fuse),
-                                   reinterpret_cast<volatile int*>(nvs)[10], warp, lane, ix0, iy0, bt, p);
+  if (FUSE && tf.out && mine) {
+    const int2 fr = tf.slab_tab[bz];
+    bp_fused_thicken<CPW, SL, CPG>(tf, vals, tf.tab + fr.x, fr.y - fr.x, warp, lane, ix0, iy0, bt, p);
+  }
   if (COUNT) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
@@ -681,8 +737,9 @@ constexpr int bp_min_ctas() {
 }
 
 // One tile per CTA: grid (tiles x, tiles y, SL-slice slabs x chunks of angles);
-// the chunks of a tile are a cluster along z.
-template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT>
+// the chunks of a tile are a cluster along z (RANGE = BP_CLUSTER; one chunk:
+// BP_ALL, whose loop bounds need no registers).
+template <typename T, int CPW, int CU, int NW, int SL, bool ZC, bool COUNT, int RANGE>
 __global__ void __launch_bounds__((NW + 1) * 32, bp_min_ctas<NW, CU, SL>())
 k_bp_tma(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, const float2* __restrict__ view_sc,
          const float* __restrict__ view_z, const float* __restrict__ zslices, BPParams p, BPTile bt,
@@ -691,10 +748,9 @@ k_bp_tma(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, const
   // it starts at the (128-byte aligned) base of the CTA's window
   extern __shared__ __align__(128) uint8_t smem[];
   bp_init_barriers(smem, NW);
-  const int chunk = (int)blockIdx.z % bt.nc;
-  bp_tile<T, CPW, CU, NW, SL, ZC, COUNT, true>(&map, vol, view_sc, view_z, zslices, p, bt, blockIdx.x, blockIdx.y,
-                                 bt.zb0 + (int)blockIdx.z / bt.nc, count, err, smem, 0u, tf,
-                                 bp_chunk_begin(chunk, bt.nc, p.P2), bp_chunk_begin(chunk + 1, bt.nc, p.P2), false);
+  const int z = (int)blockIdx.z, nc = RANGE == BP_CLUSTER ? bt.nc : 1;
+  bp_tile<T, CPW, CU, NW, SL, ZC, COUNT, true, RANGE>(&map, vol, view_sc, view_z, zslices, p, bt, blockIdx.x,
+                                                      blockIdx.y, bt.zb0 + z / nc, count, err, smem, 0u, tf, z % nc, nc);
 }
 
 // The same on the reference layout's rows (transposed, rows_to_channels), with
@@ -706,12 +762,11 @@ k_bp_tma_refq(const __grid_constant__ CUtensorMap map, float* __restrict__ vol, 
               unsigned long long* __restrict__ count, int* __restrict__ err) {
   extern __shared__ __align__(128) uint8_t smem[];
   bp_init_barriers(smem, NW);
-  const int chunk = (int)blockIdx.z % bt.nc;
   ThickFuse none;
   none.out = nullptr;
-  bp_tile<float, CPW, CU, NW, SL, false, COUNT, true, true>(
+  bp_tile<float, CPW, CU, NW, SL, false, COUNT, true, BP_CLUSTER, true>(
       &map, vol, view_sc, view_z, zslices, p, bt, blockIdx.x, blockIdx.y, (int)blockIdx.z / bt.nc, count, err, smem, 0u,
-      none, bp_chunk_begin(chunk, bt.nc, p.P2), bp_chunk_begin(chunk + 1, bt.nc, p.P2), false);
+      none, (int)blockIdx.z % bt.nc, bt.nc);
 }
 
 // out[view][channel][row] (rows padded to nrp, the padding not written) from
@@ -766,9 +821,9 @@ k_bp_tma_batch(const BpScan* __restrict__ scans, const int4* __restrict__ items,
     const BPParams p = sd->p;
     const BPTile bt = sd->bt;
     float* vol = sd->vol + (size_t)chunk * p.nz * p.ny * p.nx;
-    ring += (uint32_t)bp_tile<T, CPW, CU, NW, SL, ZC, false, false>(
+    ring += (uint32_t)bp_tile<T, CPW, CU, NW, SL, ZC, false, false, BP_ITEM>(
         &sd->map, vol, sd->view_sc, sd->view_z, sd->zslices, p, bt, w.y, w.z, w.w, nullptr, err, smem, ring, sd->tf,
-        bp_chunk_begin(chunk, nc, p.P2), bp_chunk_begin(chunk + 1, nc, p.P2), nc > 1);
+        chunk, nc);
     __syncthreads();  // the tile's shared memory and words[9] are free again
   }
 }
@@ -812,7 +867,9 @@ cudaError_t launch_one(const CUtensorMap& map, float* vol, const float2* sc,
   if (bt.zb0 < 0 || bt.zb0 >= nslab || bt.nzb < 0 || bt.zb0 + bt.nzb > nslab) return cudaErrorInvalidValue;
   dim3 grid((unsigned)((p.nx + bt.tx - 1) / bt.tx), (unsigned)((p.ny + bt.ty - 1) / bt.ty),
             (unsigned)((bt.nzb ? bt.nzb : nslab - bt.zb0) * bt.nc));
-  auto kern = count ? k_bp_tma<T, CPW, CU, NW, SL, ZC, true> : k_bp_tma<T, CPW, CU, NW, SL, ZC, false>;
+  auto kern = count       ? k_bp_tma<T, CPW, CU, NW, SL, ZC, true, BP_CLUSTER>
+              : bt.nc > 1 ? k_bp_tma<T, CPW, CU, NW, SL, ZC, false, BP_CLUSTER>
+                          : k_bp_tma<T, CPW, CU, NW, SL, ZC, false, BP_ALL>;
   cudaError_t e = prepare_kernel<NW>(kern, bt.smem_bytes);
   if (e != cudaSuccess) return e;
   return launch_cluster(kern, grid, (NW + 1) * 32, bt.smem_bytes, bt.nc, s, map, vol, sc, vz, zs, p, bt, count, err, tf);

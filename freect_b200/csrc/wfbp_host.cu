@@ -285,8 +285,8 @@ void mixed_scale_ptrs(const wfbp_ctx* ctx, P rebinned, float** row_sc, float** v
 // can reach a slab. Returns false if no configuration fits in shared
 // memory (the generic kernel is used then).
 // Slab-level view reach and the most views of one theta~ that can reach a
-// 32-slice slab (a bound for 16-slice slabs too); both depend only on the
-// geometry and the table positions.
+// slab of 16 or 32 slices; both depend only on the geometry and the table
+// positions.
 void bp_reach(wfbp_ctx* ctx, const std::vector<float>& table) {
   const double R = ctx->cg.distance_source_to_isocenter;
   const double rmax = 0.5 * ctx->cg.acquisition_field_of_view;
@@ -294,23 +294,25 @@ void bp_reach(wfbp_ctx* ctx, const std::vector<float>& table) {
   // |z - z_j| <= |A| + l_hat tan for any valid (voxel, view); tighter than z_rot
   const double cone = (R + rmax) * tanc + (ctx->cg.z_rot / (2 * M_PI)) * asin(std::min(1.0, rmax / R));
   const double reach = std::min((double)ctx->cg.z_rot, cone) + 1e-3 * (1.0 + fabs(ctx->cg.z_rot));
-  int nv_max = 0;
-  const int nslab = (ctx->nz + 31) / 32;
-  for (int sl = 0; sl < nslab; sl++) {
-    float zmn = 3e38f, zmx = -3e38f;
-    for (int i = sl * 32; i < std::min(ctx->nz, sl * 32 + 32); i++) {
-      zmn = std::min(zmn, ctx->z_native[i]);
-      zmx = std::max(zmx, ctx->z_native[i]);
-    }
-    const float lo = zmn - (float)reach, hi = zmx + (float)reach;
-    for (int t = 0; t < ctx->P2; t++) {
-      int n = 0;
-      for (int k = 0; k < ctx->K; k++) {
-        const float zt = table[t + k * ctx->P2];
-        if (!(zt < lo || zt > hi)) n++;
+  for (int slab = 16; slab <= 32; slab += 16) {
+    int nv_max = 1;
+    for (int s0 = 0; s0 < ctx->nz; s0 += slab) {
+      float zmn = 3e38f, zmx = -3e38f;
+      for (int i = s0; i < std::min(ctx->nz, s0 + slab); i++) {
+        zmn = std::min(zmn, ctx->z_native[i]);
+        zmx = std::max(zmx, ctx->z_native[i]);
       }
-      nv_max = std::max(nv_max, n);
+      const float lo = zmn - (float)reach, hi = zmx + (float)reach;
+      for (int t = 0; t < ctx->P2; t++) {
+        int n = 0;
+        for (int k = 0; k < ctx->K; k++) {
+          const float zt = table[t + k * ctx->P2];
+          if (!(zt < lo || zt > hi)) n++;
+        }
+        nv_max = std::max(nv_max, n);
+      }
     }
+    (slab == 16 ? ctx->bp_nv_max16 : ctx->bp_nv_max) = nv_max;
   }
   ctx->bp_reach = (float)reach;
   // the channel window of the default shape's 8 x 16 columns (size_bp_tile)
@@ -318,7 +320,6 @@ void bp_reach(wfbp_ctx* ctx, const std::vector<float>& table) {
   const double window = ceil(hypot(7 * vx, 15 * vy) * ctx->gp.pixel_scale) + 5.0;
   ctx->bp_nc = bp_theta_chunks(ctx->nx, ctx->ny, ctx->nz_config, ctx->P2,
                                (size_t)std::min(window, 1.0e6) * ((ctx->nr + 3) / 4 * 4) * 4);
-  ctx->bp_nv_max = std::max(1, nv_max);
   // A sample with its row in [0, nr - 2] has |z - z_j| <= cone; below z_rot
   // by a margin for rounding, the cull of cuda_kernels.cuh:232 never removes
   // one and the backprojection's records drop its row range
@@ -342,7 +343,7 @@ bool size_bp_tile(const wfbp_ctx* ctx, int tx, int ty, int cu, int nw, int slab,
   if (ext * ctx->gp.pixel_scale > 250.0) return false;  // a TMA box holds at most 256 channels
   b.W = (int)ceil(ext * ctx->gp.pixel_scale) + 5;
   b.nrp = (ctx->nr + 3) / 4 * 4;
-  b.nv_max = ctx->bp_nv_max;
+  b.nv_max = slab == 16 ? ctx->bp_nv_max16 : ctx->bp_nv_max;
   b.slot_bytes = (int)((b.W * b.nrp * 4 + 127) / 128 * 128);
   b.reach = ctx->bp_reach;
   b.smem_bytes = 0;
@@ -370,13 +371,24 @@ bool slab_allowed(const wfbp_ctx* ctx, int slab) { return ctx->ext.bp_slab == 0 
 // warps, and a 16-slice slab keeps more lanes inside a view's cone than a
 // 32-slice one, so: 8 x 16 columns / 8 warps / 16 slices where three CTAs fit an
 // SM (24 consumer warps), else 16 x 20 / 20 / 16 (20 warps in one CTA: wide view
-// windows, as a flying focal spot's), else the first candidate that fits.
-// Measured, ms, 16x16/4w16s32 (the first candidate) -> this rule: 16 rows 256 x
-// 256 x 26 FP32 7.93 -> 5.44; 20 rows 333 x 287 x 74 mixed 24.3 -> 17.9; 64 rows
-// 512 x 512 x 480 FP32 217.5 -> 200.5, mixed 206.9 -> 200.6; flying focal spot
-// 512 x 512 x 166 FP32 48.0 -> 46.6, where 8x16/8w8s16 (two CTAs) takes 68.1.
-bool default_bp_tile(const wfbp_ctx* ctx, BPTile* out) {
+// windows, as a flying focal spot's), else the first candidate that fits. With
+// the mixed form's pairs and a cone of 48 slices or more the lanes' view lists
+// fill a 32-slice slab as well, and its geometry records serve twice the lanes:
+// 8 x 16 / 8 / 32 where two CTAs fit, else 16 x 16 / 16 / 32. Measured, ms, 16-slice
+// shape / 32-slice shape: 64 rows 512 x 512 x 96 mixed 39.4 / 38.2, FP32 39.5 /
+// 39.7; flying focal spot (64 effective rows) 512 x 512 x 166 mixed 43.6 / 40.7,
+// FP32 47.4 / 47.3; 32 rows mixed 7.0 / 8.0; 20 rows mixed 15.4 / 17.3; 16 rows
+// mixed 4.64 / 5.04. 8 x 16 / 8 / 16 in two CTAs instead of 16 x 20 / 20 / 16: flying
+// focal spot FP32 70.5 against 47.4.
+bool default_bp_tile(const wfbp_ctx* ctx, bool pairs, BPTile* out) {
   BPTile b;
+  if (pairs && ctx->nr >= 48 && slab_allowed(ctx, 32) && ctx->nz > 16) {
+    if (size_bp_tile(ctx, 8, 16, 8, 8, 32, &b) && 2 * (b.smem_bytes + 1024) <= 228 * 1024) {
+      *out = b;
+      return true;
+    }
+    if (size_bp_tile(ctx, 16, 16, 8, 16, 32, out)) return true;
+  }
   if (!slab_allowed(ctx, 16)) return false;
   if (size_bp_tile(ctx, 8, 16, 8, 8, 16, &b) && 3 * (b.smem_bytes + 1024) <= 228 * 1024) {
     *out = b;
@@ -394,7 +406,7 @@ void choose_refq_tile(wfbp_ctx* ctx) {
   wfbp_ext any = ctx->ext;
   any.bp_slab = 0;  // restricts the backprojection layout's shapes only
   std::swap(ctx->ext, any);
-  const bool fits = default_bp_tile(ctx, &b) || size_bp_tile(ctx, 8, 8, 4, 16, 32, &b);
+  const bool fits = default_bp_tile(ctx, false, &b) || size_bp_tile(ctx, 8, 8, 4, 16, 32, &b);
   std::swap(ctx->ext, any);
   if (!fits || !bp_refq_supported(b)) return;
   b.zc = 0;
@@ -406,7 +418,7 @@ void choose_refq_tile(wfbp_ctx* ctx) {
 bool choose_bp_tile(wfbp_ctx* ctx, const std::vector<float>& table) {
   bp_reach(ctx, table);
   choose_refq_tile(ctx);
-  if (default_bp_tile(ctx, &ctx->bpt)) return true;
+  if (default_bp_tile(ctx, ctx->ext.precision == WFBP_PRECISION_MIXED, &ctx->bpt)) return true;
   for (auto& c : kBpCandidates) {
     if (!slab_allowed(ctx, c[4])) continue;
     BPTile b;

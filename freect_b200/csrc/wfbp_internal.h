@@ -90,12 +90,23 @@ constexpr int WFBP_ERRBIT_F16_RANGE = 0x800;  // filter: |filtered row / pair_sc
 // function sizes the launch on the host and carves the buffer on the device.
 constexpr int BT_CWARPS = 16;  // default consumer warps of the TMA backprojection
 constexpr int BT_STAGES = 2;   // view-window ring depth
-constexpr int BT_FUSE_WORDS = 384;  // shared-memory words for one slab's fused-thickening records
+constexpr int BT_FUSE_WORDS = 384;  // most words of one slab's fused-thickening records
 constexpr int BP_GEO_BYTES_ZCULL = 48;  // column-pair record with the row range of the table-position cull
 constexpr int BP_GEO_BYTES = 32;        // column-pair record when that cull never binds
+constexpr int BP_LIST_VIEWS = 14;  // most views of a stage that a lane's list of 4-bit indices can name
 struct BpSmem {
-  unsigned slots, vinfo, vgeo, geo, fuse, part, total;
+  unsigned slots, vinfo, vgeo, vwin, list, zero, geo, part, total;
 };
+// Column-pair records of one warp: [view 0 .. nv_max][column group][pair]; the
+// last view is the idle record of lanes whose list has ended. A group's records
+// are padded so that the lanes of both groups, and of different views, read
+// theirs from different banks.
+__host__ __device__ constexpr unsigned bp_geo_group(int cpw, int slab, int rec) {
+  return (unsigned)(cpw / 2 / (32 / slab) * rec + (slab == 32 ? 0 : 16));
+}
+__host__ __device__ constexpr unsigned bp_geo_view(int cpw, int slab, int rec) {
+  return (unsigned)(32 / slab) * bp_geo_group(cpw, slab, rec) + (slab == 32 ? 16u : 0u);
+}
 // Per staged view, the geometry the consumers' record pass reads (copied by
 // the producer lane that selects the view): sin and cos of the tube angle and
 // the table position, FP64 (mixed form) or FP32 (the first three floats).
@@ -113,11 +124,16 @@ __host__ __device__ inline BpSmem bp_smem_layout(const BPTile& bt, int cpw) {
   o += (unsigned)(BT_STAGES * bt.nv_max * 8);
   o = (o + 15u) & ~15u;
   L.vgeo = o;
-  o += (unsigned)(BT_STAGES * bt.nv_max * sizeof(BpViewGeo));
+  o += (unsigned)((BT_STAGES * bt.nv_max + 1) * sizeof(BpViewGeo));
+  L.vwin = o;  // float2 [nv_max] slice range of each staged view
+  o += (unsigned)(bt.nv_max * 8);
+  L.list = o;  // [STAGES][32] the lanes' views
+  o += (unsigned)(BT_STAGES * 32 * 4);
+  o = (o + 15u) & ~15u;
+  L.zero = o;  // the idle record's samples
+  o += (unsigned)(2 * bt.nrp * 4);
   L.geo = o;
-  o += (unsigned)(bt.nw * bt.nv_max * (cpw / 2) * (bt.zc ? BP_GEO_BYTES_ZCULL : BP_GEO_BYTES));  // column-pair records
-  L.fuse = o;
-  o += (unsigned)(BT_FUSE_WORDS * 4);  // the slab's fused-thickening records (ThickFuse)
+  o += (unsigned)(bt.nw * (bt.nv_max + 1)) * bp_geo_view(cpw, bt.slab, bt.zc ? BP_GEO_BYTES_ZCULL : BP_GEO_BYTES);
   // a cluster's chunk sums [warp][column][lane]: over the ring when they fit there (it is idle by then)
   L.part = L.slots;
   if (bt.nc > 1) {
@@ -232,7 +248,8 @@ struct wfbp_ctx {
   BPTile bpt;
   float bp_reach = 0.0f;            // slab-level view prefilter half width (mm)
   int bp_nc = 1;                    // chunks of half-turn angles (bp_theta_chunks)
-  int bp_nv_max = 1;                // most views of one theta~ reaching a slab
+  int bp_nv_max = 1;                // most views of one theta~ reaching a 32-slice slab
+  int bp_nv_max16 = 1;              // ... a 16-slice slab
   int bp_zcull = 1;                 // 0: the table-position cull (|z - z_j| > z_rot) never removes a
                                     // sample whose row lies in [0, nr - 2] (cone shorter than z_rot)
 
