@@ -517,19 +517,26 @@ __device__ __forceinline__ float rebin_view_weight(int v, int y, float beta, flo
   return w;
 }
 
-// One thread per raw sample (reading y, raw row, raw channel).
-__global__ void k_rebin_adjoint(const float* __restrict__ gR, float* __restrict__ graw, const float* __restrict__ beta_t,
-                                const int* __restrict__ cnt, const int* __restrict__ cidx, const float* __restrict__ cw,
-                                int maxl, RebinParams p) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long total = (long)p.V * p.nr * p.nch;
-  if (i >= total) return;
-  const int xr = (int)(i % p.nch);
-  const int rr = (int)((i / p.nch) % p.nr);
-  const int y = (int)(i / ((long)p.nch * p.nr));
-  const int x = p.nch - 1 - xr;   // sheet column
-  const int row = p.nr - 1 - rr;  // sheet row index i of the output
-  float acc = 0.0f;
+// One thread per raw channel of a reading and RA_ROWS of its detector rows: the
+// view weights of a channel do not depend on the row, so they are computed
+// once, and the rows' independent loads hide each other's latency (a thread
+// per sample spent its time on the weights: 16 rows of 672 channels 1.03 ms,
+// now 0.37; 64 rows of 888 channels, 2460 readings, 3.66 ms, now 1.00, of
+// which moving its 1.1 GB takes 0.17). Lanes are consecutive raw channels,
+// whose sources are consecutive channels.
+constexpr int RA_ROWS = 8, RA_CH = 128;
+
+__global__ void __launch_bounds__(RA_CH)
+k_rebin_adjoint(const float* __restrict__ gR, float* __restrict__ graw, const float* __restrict__ beta_t,
+                const int* __restrict__ cnt, const int* __restrict__ cidx, const float* __restrict__ cw, int maxl,
+                RebinParams p) {
+  const int y = blockIdx.x, xr = blockIdx.y * RA_CH + threadIdx.x, i0 = blockIdx.z * RA_ROWS;
+  if (xr >= p.nch) return;
+  const int x = p.nch - 1 - xr;  // sheet column
+  const int rows = min(RA_ROWS, p.nr - i0);  // sheet rows i0 .. of the output
+  float acc[RA_ROWS];
+#pragma unroll
+  for (int k = 0; k < RA_ROWS; k++) acc[k] = 0.0f;
   const int n = cnt[x];
   for (int e = 0; e < n; e++) {
     const int c = cidx[x * maxl + e];
@@ -543,14 +550,25 @@ __global__ void k_rebin_adjoint(const float* __restrict__ gR, float* __restrict_
     if (y == p.V - 1) v_lo = min(v_lo, (int)floorf((float)(p.V - 1) + sh) - 2);
     v_lo = max(v_lo, 0);
     v_hi = min(v_hi, p.V - 1);
-    float sum = 0.0f;
+    float sum[RA_ROWS];
+#pragma unroll
+    for (int k = 0; k < RA_ROWS; k++) sum[k] = 0.0f;
     for (int v = v_lo; v <= v_hi; v++) {
       const float wy = rebin_view_weight(v, y, beta, p.dth, p.V, p.q8, p.voff);
-      if (wy != 0.0f) sum = fmaf(wy, __ldg(gR + ((size_t)v * p.nr + row) * p.nch + c), sum);
+      if (wy == 0.0f) continue;
+      const float* g = gR + ((size_t)v * p.nr + i0) * p.nch + c;
+#pragma unroll
+      for (int k = 0; k < RA_ROWS; k++)
+        if (k < rows) sum[k] = fmaf(wy, __ldg(g + (size_t)k * p.nch), sum[k]);
     }
-    acc = fmaf(wx, sum, acc);
+#pragma unroll
+    for (int k = 0; k < RA_ROWS; k++) acc[k] = fmaf(wx, sum[k], acc[k]);
   }
-  graw[i] = acc;
+  // sheet row i is raw row nr - 1 - i
+  float* out = graw + ((size_t)y * p.nr + (p.nr - 1 - i0)) * p.nch + xr;
+#pragma unroll
+  for (int k = 0; k < RA_ROWS; k++)
+    if (k < rows) out[-(ptrdiff_t)k * p.nch] = acc[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -741,8 +759,8 @@ cudaError_t launch_rebin_adj_cols(const float* bidx, int nch, int q8, int* cnt, 
 
 cudaError_t launch_rebin_adjoint(const float* gR, float* graw, const float* beta, const int* cnt, const int* cidx,
                                  const float* cw, int maxl, const RebinParams& p, cudaStream_t s) {
-  const long n = (long)p.V * p.nr * p.nch;
-  k_rebin_adjoint<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gR, graw, beta, cnt, cidx, cw, maxl, p);
+  const dim3 g((unsigned)p.V, (unsigned)((p.nch + RA_CH - 1) / RA_CH), (unsigned)((p.nr + RA_ROWS - 1) / RA_ROWS));
+  k_rebin_adjoint<<<g, RA_CH, 0, s>>>(gR, graw, beta, cnt, cidx, cw, maxl, p);
   return cudaGetLastError();
 }
 
