@@ -801,7 +801,7 @@ k_rows_to_channels(const T* __restrict__ in, const float* __restrict__ scales, f
 
 // Persistent launch over the column tiles of several scans: each CTA takes
 // the next work item (scan | chunk of angles << 24, tile x, tile y, slab) from
-// a global counter until the list is exhausted. Items are listed by decreasing estimated cost.
+// a global counter until the list is exhausted.
 template <typename T, int CPW, int CU, int NW, int SL, bool ZC>
 __global__ void __launch_bounds__((NW + 1) * 32, bp_min_ctas<NW, CU, SL, true>())
 k_bp_tma_batch(const BpScan* __restrict__ scans, const int4* __restrict__ items, int n_items,

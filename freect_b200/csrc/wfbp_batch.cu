@@ -5,16 +5,18 @@
 // Per scan the rebin and filter stages run as their own launches (their
 // shapes differ from scan to scan); the backprojection of all scans is ONE
 // persistent launch (k_bp_tma_batch) whose CTAs take work items -- a column
-// tile and slab (32 or 16 native slices) of one scan -- from a list sorted by estimated
-// cost, so uneven scans share the GPU without a tail per scan; thickening is
-// again per scan. The whole chain is captured once into a CUDA graph and
-// replayed while the caller's input and output pointers stay the same.
+// tile, slab (32 or 16 native slices) and chunk of half-turn angles of one
+// scan -- from one list, so uneven scans share the GPU without a tail per
+// scan; thickening is again per scan. The whole chain is captured once into a
+// CUDA graph and replayed while the caller's input and output pointers stay
+// the same.
 #include "wfbp_internal.h"
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #define WFBP_API extern "C" __attribute__((visibility("default")))
@@ -40,7 +42,7 @@ struct wfbp_batch {
   cudaGraphExec_t exec = nullptr;
   std::vector<const void*> key;
   std::string err;
-  std::vector<int4> h_items;          // the cost-sorted work list (host copy)
+  std::vector<int4> h_items;          // the work list (host copy)
   // wfbp_batch_run_host: device copies of the readings and volumes, the copy
   // stream and its events, and the work list split into two launches
   std::vector<float*> raw_d, vol_d;
@@ -115,7 +117,7 @@ std::vector<double> slab_view_counts(const wfbp_ctx* c, const std::vector<float>
 }
 
 // Lays out the persistent launch for configuration b->cfg: per-scan launch
-// sizes, tensor maps and the cost-sorted work list.
+// sizes, tensor maps and the work list.
 int build_plan(wfbp_batch* b) {
   const int n = (int)b->ctx.size();
   std::vector<BpScan> hs(n);
@@ -183,7 +185,19 @@ int build_plan(wfbp_batch* b) {
             items.push_back({make_int4(i | ch << 24, bx, by, sl), ((double)cols * nv[sl] + 1.0) / c->bp_nc});
       }
   }
-  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& c) { return a.cost > c.cost; });
+  // Scan by scan, the one with the largest items first (the launch ends on
+  // small ones), each in the order of a launch of its own: CTAs that run
+  // together then stage the same views' neighbouring windows, which stay in
+  // L2. Sorted by cost over all scans the list was 1 % slower (four scans of 32
+  // rows 24.5 -> 24.2 ms FP32, 22.2 -> 21.9 mixed; 24 scans of 16 to 64 rows
+  // 1391 -> 1374 ms), in classes of equal log2 cost as slow as by cost.
+  std::vector<double> top(n, 0.0);
+  for (const Item& it : items) top[it.w.x & 0xffffff] = std::max(top[it.w.x & 0xffffff], it.cost);
+  std::stable_sort(items.begin(), items.end(), [&](const Item& a, const Item& c) {
+    const int sa = a.w.x & 0xffffff, sc = c.w.x & 0xffffff;
+    if (sa != sc) return top[sa] != top[sc] ? top[sa] > top[sc] : sa < sc;
+    return std::make_tuple(a.w.w, a.w.z, a.w.y, a.w.x) < std::make_tuple(c.w.w, c.w.z, c.w.y, c.w.x);
+  });
   std::vector<int4> hw(items.size());
   for (size_t k = 0; k < items.size(); k++) hw[k] = items[k].w;
   free_plan(b);
@@ -492,7 +506,7 @@ WFBP_API int wfbp_batch_run_host(wfbp_batch* b, const float* const* raws_host, f
     std::vector<int4> split;
     split.reserve(b->h_items.size());
     for (const int4& w : b->h_items)
-      if ((w.x & 0xffffff) < k) split.push_back(w);  // stable: each group keeps the cost order
+      if ((w.x & 0xffffff) < k) split.push_back(w);  // stable: each group keeps the order
     const int na = (int)split.size();
     for (const int4& w : b->h_items)
       if ((w.x & 0xffffff) >= k) split.push_back(w);
