@@ -33,27 +33,19 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "backproj voxel-view updates/s & s/volume at <=1 HU RMSE vs FP64; mixed vs FP32"
-# DRAM read + write bytes and warp instructions per contributing update of one backprojection
-# launch, from the ncu captures of rows64_short (2.3819501378e10 updates; profiles/
-# k_bp_tma_rows64_short.md), by precision form and slab height (16-slice slabs stage each view
-# window in twice as many CTAs); the kernel's binding limit is instruction issue
-# ncu captures of k_bp_tma on rows64_short (2.3819501378e10 updates per launch;
-# profiles/k_bp_tma_rows64_short.md): DRAM bytes and warp instructions per
-# update, keyed by (form, configuration) for the shapes the autotuner picks on
-# rows64, else by (form, slab height)
+# DRAM read + write bytes and warp instructions per contributing update of one k_bp_tma launch,
+# from the ncu captures of rows64_short (profiles/k_bp_tma_rows64_short.md), keyed by (form,
+# configuration) for the shapes the autotuner picks on rows64, else by (form, slab height);
+# ("fp32", 32) and ("mixed", 16) are captures from before the view lists
 _SHORT_UPDATES = 2.3819501378e10
-DRAM_BYTES_PER_UPDATE = {("fp32", 32): 14.42e9 / _SHORT_UPDATES,
-                         ("mixed", 16): 14.39e9 / _SHORT_UPDATES,
-                         ("fp32", 16): 21.08e9 / _SHORT_UPDATES,
-                         ("mixed", 32): 13.18e9 / _SHORT_UPDATES,
-                         ("mixed", "16x8/4w8s16"): 34.96e9 / _SHORT_UPDATES,
-                         ("fp32", "16x8/8w8s32"): 15.38e9 / _SHORT_UPDATES,
-                         ("fp32", "8x16/8w8s16"): 22.55e9 / _SHORT_UPDATES}
-WARP_INST_PER_UPDATE = {("fp32", 32): 3.537e10 / _SHORT_UPDATES, ("mixed", 16): 3.428e10 / _SHORT_UPDATES,
-                        ("fp32", 16): 3.475e10 / _SHORT_UPDATES, ("mixed", 32): 3.631e10 / _SHORT_UPDATES,
-                        ("mixed", "16x8/4w8s16"): 3.6336e10 / _SHORT_UPDATES,
-                        ("fp32", "16x8/8w8s32"): 3.4076e10 / _SHORT_UPDATES,
-                        ("fp32", "8x16/8w8s16"): 3.4219e10 / _SHORT_UPDATES}
+DRAM_BYTES_PER_UPDATE = {("mixed", "8x16/8w8s32"): 10.88e9 / _SHORT_UPDATES,
+                         ("fp32", "8x16/8w8s16"): 22.79e9 / _SHORT_UPDATES,
+                         ("mixed", 32): 10.88e9 / _SHORT_UPDATES, ("fp32", 16): 22.79e9 / _SHORT_UPDATES,
+                         ("fp32", 32): 15.38e9 / _SHORT_UPDATES, ("mixed", 16): 34.96e9 / _SHORT_UPDATES}
+WARP_INST_PER_UPDATE = {("mixed", "8x16/8w8s32"): 3.1603e10 / _SHORT_UPDATES,
+                        ("fp32", "8x16/8w8s16"): 3.3912e10 / _SHORT_UPDATES,
+                        ("mixed", 32): 3.1603e10 / _SHORT_UPDATES, ("fp32", 16): 3.3912e10 / _SHORT_UPDATES,
+                        ("fp32", 32): 3.4076e10 / _SHORT_UPDATES, ("mixed", 16): 3.6336e10 / _SHORT_UPDATES}
 SMS, SCHEDULERS_PER_SM = 148, 4
 UNIT = "voxel-view updates/s"
 
@@ -654,7 +646,9 @@ def main():
         # the batched uneven scans (24 scans, one persistent launch): the batch
         # autotuner tries the three fastest rows64 mixed shapes that fit
         tms = head["tuning"] or {}
-        cands = sorted(tms, key=tms.get)[:3] if tms else None
+        # the two fastest shapes of each slab height: the better height depends on a scan's detector rows
+        cands = [k for h in ("s32", "s16") for k in sorted((t for t in tms if t.endswith(h)), key=tms.get)[:2]]
+        cands = cands or None
         try:
             line["batch24"] = measure_batch(args, rank, world, local, dist, candidates=cands,
                                             hu_scans=args.batch_hu_scans, steps=min(args.steps, 3), warmup=1)
@@ -716,8 +710,9 @@ def stage_rooflines(form, ctx, d, updates, stage, clk):
     rebin: HBM, raw frames read once + rebinned output written once.
     filter: tensor pipe (mixed: 3 split-FP16 products of 2 (V nr) nch^2
     FLOP each, against the sustained cuBLAS BF16 rate, the same tensor rate
-    as FP16) or FP32 FFMA (FP32
-    form: 2 (V nr) nch^2 FLOP against 148 SMs x 128 lanes x 2 x clock)."""
+    as FP16); FP32 form: HBM (FFT, rows read and written once), beyond 2047
+    channels FP32 FFMA (2 (V nr) nch^2 FLOP against 148 SMs x 128 lanes x 2 x
+    clock)."""
     hbm, bf16, bf16_sus, peak_src = load_peaks()
     mhz = (clk or {}).get("sm_mhz") or 1965.0
     bpc = ctx.bp_config()
@@ -756,6 +751,10 @@ def stage_rooflines(form, ctx, d, updates, stage, clk):
                 "unit": "TFLOP/s", "frac": flop / t_f / 1e12 / bf16_sus, "algorithmic_flop": flop,
                 "note": "3 split-FP16 products (hi*hi, hi*lo, lo*hi) of 2 M K N, M = views x rows, K = N = "
                         "channels, against the sustained cuBLAS BF16 rate (FP16 runs at the same tensor rate)"}
+    elif d.n_channels < 2048:  # k_filter_fft
+        filt = {"bound": "hbm", "kernel": "filter_fft", "achieved": samples * 8 / t_f / 1e9, "peak": hbm, "unit": "GB/s",
+                "frac": samples * 8 / t_f / 1e9 / hbm, "algorithmic_bytes": samples * 8,
+                "note": "FP32 FFT filter: rows read once and written once, 4 B a sample"}
     else:
         flop = 2.0 * rows * d.n_channels * d.n_channels
         fpk = SMS * 128 * 2 * mhz * 1e6 / 1e12
@@ -763,9 +762,9 @@ def stage_rooflines(form, ctx, d, updates, stage, clk):
                 "unit": "TFLOP/s", "frac": flop / t_f / 1e12 / fpk, "algorithmic_flop": flop,
                 "note": "FP32 FFMA Toeplitz, peak = 148 SMs x 128 lanes x 2 FLOP x sampled clock"}
     for r in (bp, rebin, filt):
-        r["peak_source"] = peak_src if r is not filt or form == "mixed" else "nominal"
+        r["peak_source"] = "nominal" if r["bound"] == "fp32" else peak_src
         r["ms"] = {"backproject": stage["backproject"], "rebin": stage["rebin"], "toeplitz_tc": stage["filter"],
-                   "toeplitz_f32": stage["filter"]}[r["kernel"]]
+                   "filter_fft": stage["filter"], "toeplitz_f32": stage["filter"]}[r["kernel"]]
     return bp, {"backproject": bp, "rebin": rebin, "filter": filt}
 
 

@@ -1293,7 +1293,7 @@ WFBP_API int wfbp_backproject_adjoint(wfbp_ctx* ctx, const float* g_native, floa
   // time, refilled in every call. A refilled table costs a weight sum per
   // (voxel, angle, slice) and a pass over it, the gather without a table a sum
   // per (voxel, view, slice) with all its views' geometry (64 rows, 256 x 256 x
-  // 64: 10 against 270 ms), so that form is left to memory too small for one
+  // 64: 8.5 against 270 ms), so that form is left to memory too small for one
   // angle's weights.
   const size_t per_angle = (size_t)ctx->nz * ctx->nx * ctx->ny;
   int angles = (int)std::min<size_t>(ctx->P2, kAdjointTableBytes / sizeof(float) / per_angle);
