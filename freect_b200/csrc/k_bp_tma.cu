@@ -338,7 +338,9 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
             const float t1 = xa * sc.y + ya * sc.x, t2 = xa * sc.y + yb * sc.x;
             const float t3 = xb * sc.y + ya * sc.x, t4 = xb * sc.y + yb * sc.x;
             const float lhi = sqrtf(p.R2) - fminf(fminf(t1, t2), fminf(t3, t4));
-            const float amin = p.zr2pi * asinf(p.rR * pmin), amax = p.zr2pi * asinf(p.rR * pmax);
+            // (a corner beyond the source's orbit: no voxel of the field has |p_hat| >= R, the clamp keeps the bound)
+            const float amin = p.zr2pi * asinf(fmaxf(p.rR * pmin, -1.0f)),
+                        amax = p.zr2pi * asinf(fminf(p.rR * pmax, 1.0f));
             const float eps = 1e-3f * (1.0f + fabsf(zt));
             wlo = zt - amax - lhi * p.tanc - eps;
             whi = zt - amin + lhi * p.tanc + eps;
