@@ -209,9 +209,9 @@ __device__ __forceinline__ void bp_fused_zero(const ThickFuse& tf, int bz, int w
 // ring before this tile (stage = ring & 1, phase = (ring >> 1) & 1), so a
 // persistent CTA continues the barriers' phases from tile to tile. The tile
 // sums the half-turn angles of chunk `chunk` of nc. With BP_CLUSTER the CTA is
-// number `chunk` of a cluster of nc that share the tile's angles: the CTAs
-// leave their sums in shared memory, and CTA r adds them in chunk order for its
-// warps w = r mod nc and writes those columns. BP_ITEM with nc > 1 writes the
+// number `chunk` of a cluster of nc that share the tile's angles: the CTAs (if
+// there are several) leave their sums in shared memory, and CTA r adds them in
+// chunk order for its warps w = r mod nc and writes those columns. BP_ITEM with nc > 1 writes the
 // plain sums (a batch's chunk).
 // Returns the number of ring steps the tile used: te - tb, or 0 for a tile entirely
 // outside the reconstruction FOV (whose voxels are written as 0, the value
@@ -419,7 +419,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
       }
     }
     __syncwarp();
-    if (RANGE == BP_CLUSTER) {  // the consumers' barriers below
+    if (RANGE == BP_CLUSTER && bp_exchanges(nc)) {  // the consumers' barriers below
       __syncthreads();
       cluster_sync();
       cluster_sync();
@@ -678,7 +678,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
   }
 
   bool mine = true;  // this CTA writes this warp's columns
-  if constexpr (RANGE == BP_CLUSTER) {
+  if (RANGE == BP_CLUSTER && bp_exchanges(nc)) {  // one chunk: its sums are complete, and the layout has no room for them
     // the chunks' sums of this warp's columns, added in chunk order
     const uint32_t part = smem_u32(smem + L.part) + (uint32_t)((warp * CPG * 32 + lane) * 4);
     __syncthreads();  // the ring is idle in this CTA

@@ -76,6 +76,9 @@ inline int bp_theta_chunks(int nx, int ny, int nz, int P2, size_t window_bytes) 
   while (nc < BP_MAX_CHUNKS && P2 >= 8 * nc && tiles * nc < (P2 >= 128 * nc ? 2 * wave : wave)) nc *= 2;
   return nc;
 }
+// The chunks' sums pass through shared memory (bp_smem_layout's part region,
+// which only such a launch has) when there are several.
+__host__ __device__ constexpr bool bp_exchanges(int nc) { return nc > 1; }
 __host__ __device__ inline int bp_chunk_begin(int chunk, int nc, int P2) { return (int)((long)P2 * chunk / nc); }
 
 // Bits of the device-side error word besides WFBP_ERR_TIMEOUT (which a
@@ -136,7 +139,7 @@ __host__ __device__ inline BpSmem bp_smem_layout(const BPTile& bt, int cpw) {
   o += (unsigned)(bt.nw * (bt.nv_max + 1)) * bp_geo_view(cpw, bt.slab, bt.zc ? BP_GEO_BYTES_ZCULL : BP_GEO_BYTES);
   // a cluster's chunk sums [warp][column][lane]: over the ring when they fit there (it is idle by then)
   L.part = L.slots;
-  if (bt.nc > 1) {
+  if (bp_exchanges(bt.nc)) {
     const unsigned bytes = (unsigned)(bt.tx * bt.ty * bt.slab) * 4u;
     if (bytes > L.vinfo - L.slots) {
       o = (o + 15u) & ~15u;
