@@ -826,6 +826,9 @@ k_bp_tma_batch(const BpScan* __restrict__ scans, const int4* __restrict__ items,
     ring += (uint32_t)bp_tile<T, CPW, CU, NW, SL, ZC, false, false, BP_ITEM>(
         &sd->map, vol, sd->view_sc, sd->view_z, sd->zslices, p, bt, w.y, w.z, w.w, nullptr, err, smem, ring, sd->tf,
         chunk, nc);
+    // The next tile's layout may be another scan's: its TMA writes can land
+    // where this tile had records, lists or sums.
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();  // the tile's shared memory and words[9] are free again
   }
 }
