@@ -659,10 +659,23 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
                                                    __saturatef(fmaf(fabsf(a.y), ka, -1.5f))),
                                        pi2);
           float2 W = __ffma2_rn(half2c, make_float2(__cosf(tt.x), __cosf(tt.y)), half2c);
-          W.x = okx ? W.x : 0.0f;
-          W.y = oky ? W.y : 0.0f;
-          ag[u2] = __ffma2_rn(W, gval, ag[u2]);
-          aw[u2] = __fadd2_rn(aw[u2], W);
+          if constexpr (REFQ) {
+            // a sample that is not the voxel's stays out altogether: times a
+            // weight of 0 one that is not finite would make the voxel NaN
+            if (okx) {
+              ag[u2].x = fmaf(W.x, gval.x, ag[u2].x);
+              aw[u2].x += W.x;
+            }
+            if (oky) {
+              ag[u2].y = fmaf(W.y, gval.y, ag[u2].y);
+              aw[u2].y += W.y;
+            }
+          } else {
+            W.x = okx ? W.x : 0.0f;
+            W.y = oky ? W.y : 0.0f;
+            ag[u2] = __ffma2_rn(W, gval, ag[u2]);
+            aw[u2] = __fadd2_rn(aw[u2], W);
+          }
           if (COUNT) cnt += (okx ? 1 : 0) + (oky ? 1 : 0);
         }
       }
