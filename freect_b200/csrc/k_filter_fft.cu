@@ -379,11 +379,16 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
     }
     if constexpr (TR) {
       float* y = Y + (size_t)v * nch * nrp + r0;  // nrp is a multiple of 4, r0 even
+      const bool both = has_b && (reinterpret_cast<uintptr_t>(Y) & 7) == 0;  // Y may be at any float
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         const int n = j * T + t;
-        if (n < nch && has_b) *reinterpret_cast<float2*>(y + (size_t)n * nrp) = a[j];
-        else if (n < nch && has_a) y[(size_t)n * nrp] = a[j].x;
+        if (n < nch && both) {
+          *reinterpret_cast<float2*>(y + (size_t)n * nrp) = a[j];
+        } else if (n < nch) {
+          if (has_a) y[(size_t)n * nrp] = a[j].x;
+          if (has_b) y[(size_t)n * nrp + 1] = a[j].y;
+        }
       }
     } else {
 #pragma unroll
