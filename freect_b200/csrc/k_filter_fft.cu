@@ -16,9 +16,12 @@
 // rounded relative to the difference: y[n] = sum_i d[i] a[n - i] with the
 // running sums a[m] = h[0] / 2 + h[1] + ... + h[m], a[-1-m] = -a[m] (the
 // constant that makes them antisymmetric meets sum d = 0). Its kernel a acts
-// like a Hilbert transform, whose spectrum is flat. Each row is scaled by the
-// power of two that brings its largest sample into [1, 2), so neither row of a
-// pair meets the other's rounding; twiddles and spectrum are rounded from FP64.
+// like a Hilbert transform, whose spectrum is flat. Both rows of a pair meet the
+// transform's rounding, which is relative to the 2-norm of what is transformed:
+// each is scaled by a power of two that brings the norm of its differences near 1
+// (a row scaled by its largest sample was, smooth beside a rough row, up to 45
+// times less exact than the Toeplitz product; by the norm it is more exact than
+// that); twiddles and spectrum are rounded from FP64.
 // A pair with a sample that is not finite or beyond 1e30 (where the
 // transform's sums could overflow although the filtered row does not) is
 // evaluated as the Toeplitz sum, sample by sample.
@@ -157,6 +160,60 @@ __device__ __forceinline__ int fft_word(int k1, int t) {
   return k1 * BLK + (t ^ chunk_xor<R3>(R2 > 1 ? t / R3 : k1));
 }
 
+// 2-norm of a row's differences: the bits of the largest magnitude (which order
+// as the magnitudes do, NaN above all) and the sum of the squares in units of
+// 2^-19 times the square of that magnitude's power of two (2048 squares below 4
+// fit 32 bits).
+struct RowNorm {
+  unsigned top, sum;
+};
+__device__ __forceinline__ unsigned top_exponent(unsigned top) { return max(top >> 23, 1u); }
+
+// Of the eight differences of each thread, over the threads of a transform, or
+// of a warp where a transform takes several.
+template <int T>
+__device__ __forceinline__ RowNorm row_norm(const float2 (&a)[8], float float2::*row) {
+  unsigned top = 0u;
+#pragma unroll
+  for (int j = 0; j < 8; j++) top = max(top, __float_as_uint(a[j].*row) & 0x7fffffffu);
+  if constexpr (T >= 32) {
+    top = __reduce_max_sync(0xffffffffu, top);
+  } else {
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  }
+  // times 2^(127 - e); a magnitude of FF_BIG or more (its row is not transformed) as it comes
+  const float s = __uint_as_float((254u - min(top_exponent(top), 253u)) << 23);
+  float q = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; j++) q = fmaf(a[j].*row * s, a[j].*row * s, q);
+  unsigned sum = (unsigned)(q * 524288.0f);
+  if constexpr (T >= 32) {
+    sum = __reduce_add_sync(0xffffffffu, sum);
+  } else {
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  }
+  return {top, sum};
+}
+
+// The norm over the warps of a transform (w at distance 2).
+template <int W>
+__device__ __forceinline__ RowNorm join_norms(const RowNorm* w) {
+  RowNorm r = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < W; i++) r.top = max(r.top, w[2 * i].top);
+#pragma unroll
+  for (int i = 0; i < W; i++)
+    r.sum += w[2 * i].sum >> min(2u * (top_exponent(r.top) - top_exponent(w[2 * i].top)), 31u);
+  return r;
+}
+
+// Biased exponent of the power of two that the norm is divided by: the norm lands in [1/2, 4).
+__device__ __forceinline__ unsigned norm_exponent(const RowNorm& r) {
+  return top_exponent(r.top) + (unsigned)(max(31 - __clz((int)r.sum) - 19, 0) >> 1);
+}
+
 // Rows of X [V][nr][nch] -> Y, rows as they are or (TR) in the backprojection
 // layout Y[view][channel][nrp]. Rows 2 i and 2 i + 1 of a view are a pair (an
 // odd view's last row is alone), so that a row's roundings do not depend on
@@ -174,7 +231,7 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
   static_assert(T == R2 * R3, "N = 16 R2 R3");
   extern __shared__ float sm_fft[];
   __shared__ float2 s_tw2[R2 * R3];       // twiddles of pass 2, [k2][n3]
-  __shared__ unsigned s_max[2][NW][2];    // row maxima of the pair by warp, two buffers
+  __shared__ RowNorm s_norm[2][NW][2];    // of the pair's rows by warp, two buffers
   const int tid = threadIdx.x, g = tid / T, t = tid % T;
   float* re = sm_fft + (size_t)g * 2 * PLANE;
   float* im = re + PLANE;
@@ -195,10 +252,9 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
     const int r0 = 2 * (int)(pair - v * per_view);
     const long m = v * nr + r0;  // row of X
     const bool has_a = pair < pairs, has_b = has_a && r0 + 1 < nr;
-    // ---- pass 1: points n = n1 T + t, n1 < 8 (the others are padding), and
+    // ---- pass 1: points n = n1 T + t, n1 < 8 (the others are padding), minus
     // their left neighbours (from L1)
-    float2 a[8], l[8];
-    unsigned ma = 0u, mb = 0u;
+    float2 a[8];
     const float *xa = X + m * nch, *xb = xa + nch;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
@@ -209,48 +265,30 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const int n = j * T + t - 1;
-      l[j].x = has_a && n >= 0 && n < nch ? __ldg(xa + n) : 0.0f;
-      l[j].y = has_b && n >= 0 && n < nch ? __ldg(xb + n) : 0.0f;
+      a[j].x -= has_a && n >= 0 && n < nch ? __ldg(xa + n) : 0.0f;
+      a[j].y -= has_b && n >= 0 && n < nch ? __ldg(xb + n) : 0.0f;
     }
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      ma = max(ma, __float_as_uint(a[j].x) & 0x7fffffffu);  // magnitudes order as their bits, NaN above all
-      mb = max(mb, __float_as_uint(a[j].y) & 0x7fffffffu);
-    }
-    if constexpr (T >= 32) {
-      ma = __reduce_max_sync(0xffffffffu, ma);
-      mb = __reduce_max_sync(0xffffffffu, mb);
-      if constexpr (T > 32) {
-        if (tid % 32 == 0) {
-          s_max[buf][tid / 32][0] = ma;
-          s_max[buf][tid / 32][1] = mb;
-        }
-        __syncthreads();  // also: the previous step's pass 1' has read its points
-#pragma unroll
-        for (int w = 0; w < T / 32; w++) {
-          ma = max(ma, s_max[buf][g * (T / 32) + w][0]);
-          mb = max(mb, s_max[buf][g * (T / 32) + w][1]);
-        }
-      } else {
-        __syncwarp();
+    RowNorm na = row_norm<T>(a, &float2::x), nb = row_norm<T>(a, &float2::y);
+    if constexpr (T > 32) {
+      if (tid % 32 == 0) {
+        s_norm[buf][tid / 32][0] = na;
+        s_norm[buf][tid / 32][1] = nb;
       }
+      __syncthreads();  // also: the previous step's pass 1' has read its points
+      na = join_norms<T / 32>(&s_norm[buf][g * (T / 32)][0]);
+      nb = join_norms<T / 32>(&s_norm[buf][g * (T / 32)][1]);
     } else {
-#pragma unroll
-      for (int o = T / 2; o > 0; o >>= 1) {
-        ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-        mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-      }
       __syncwarp();
     }
-    const bool bad = ma >= FF_BIG || mb >= FF_BIG;  // the same for all threads of the transform
+    const bool bad = na.top >= FF_BIG || nb.top >= FF_BIG;  // the same for all threads of the transform
     // powers of two: row times 2^(127 - e), result times 2^(e - 127); a row of zeros gives zeros
-    const unsigned ea = max(ma >> 23, 1u), eb = max(mb >> 23, 1u);
+    const unsigned ea = norm_exponent(na), eb = norm_exponent(nb);
     const float sa = __uint_as_float((254u - ea) << 23), sb = __uint_as_float((254u - eb) << 23);
-    const float ua = ma ? __uint_as_float(ea << 23) : 0.0f, ub = mb ? __uint_as_float(eb << 23) : 0.0f;
+    const float ua = na.top ? __uint_as_float(ea << 23) : 0.0f, ub = nb.top ? __uint_as_float(eb << 23) : 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      a[j].x = bad ? 0.0f : (a[j].x - l[j].x) * sa;
-      a[j].y = bad ? 0.0f : (a[j].y - l[j].y) * sb;
+      a[j].x = bad ? 0.0f : a[j].x * sa;
+      a[j].y = bad ? 0.0f : a[j].y * sb;
     }
     {
       float2 o[8];
