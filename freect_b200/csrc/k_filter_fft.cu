@@ -22,9 +22,13 @@
 // (a row scaled by its largest sample was, smooth beside a rough row, up to 45
 // times less exact than the Toeplitz product; by the norm it is more exact than
 // that); twiddles and spectrum are rounded from FP64.
-// A pair with a sample that is not finite or beyond 1e30 (where the
-// transform's sums could overflow although the filtered row does not) is
-// evaluated as the Toeplitz sum, sample by sample.
+// A row with a sample that is not finite or beyond 1e30 (where the transform's
+// sums could overflow although the filtered row does not), and a row of few
+// samples that are not 0 (a lone reading, the gradient of a small region), is
+// summed as the Toeplitz product sums it: the product's error grows with the root
+// of the terms, the transform's is spread over the whole row, and they cross at 25
+// samples (N = 256) to 70 (N = 2048) and 90 (N = 4096; one sample: 3e-8 of the row
+// against 1e-7). "Few" is 64, 96 from N = 1024, 128 at N = 4096.
 //
 // Two rows are one complex sequence d_a + i d_b: the kernel a is real, so the
 // inverse transform is y_a + i y_b without any unpacking. N = 16 R2 R3 points
@@ -160,20 +164,26 @@ __device__ __forceinline__ int fft_word(int k1, int t) {
   return k1 * BLK + (t ^ chunk_xor<R3>(R2 > 1 ? t / R3 : k1));
 }
 
-// 2-norm of a row's differences: the bits of the largest magnitude (which order
-// as the magnitudes do, NaN above all) and the sum of the squares in units of
-// 2^-19 times the square of that magnitude's power of two (2048 squares below 4
-// fit 32 bits).
-struct RowNorm {
-  unsigned top, sum;
-};
-__device__ __forceinline__ unsigned top_exponent(unsigned top) { return max(top >> 23, 1u); }
-
-// Of the eight differences of each thread, over the threads of a transform, or
-// of a warp where a transform takes several.
+// Sum over the threads of a transform, or of a warp where a transform takes several.
 template <int T>
-__device__ __forceinline__ RowNorm row_norm(const float2 (&a)[8], float float2::*row) {
-  unsigned top = 0u;
+__device__ __forceinline__ unsigned reduce_add(unsigned v) {
+  if constexpr (T >= 32) return __reduce_add_sync(0xffffffffu, v);
+#pragma unroll
+  for (int o = T / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The power of two (biased exponent) that a row is divided by, from its eight
+// differences in each thread: that of their 2-norm over the threads of a
+// transform, or of a warp where a transform takes several (the row takes its
+// warps' largest: at most sqrt(8) below its norm's); FF_OUT where a difference is
+// not finite or FF_BIG or more. some: the thread's samples that are not 0 in, the
+// transform's or warp's out.
+constexpr unsigned FF_OUT = 255u;
+
+template <int T>
+__device__ __forceinline__ unsigned row_exponent(const float2 (&a)[8], float float2::*row, unsigned& some) {
+  unsigned top = 0u;  // magnitudes order as their bits, NaN above all
 #pragma unroll
   for (int j = 0; j < 8; j++) top = max(top, __float_as_uint(a[j].*row) & 0x7fffffffu);
   if constexpr (T >= 32) {
@@ -182,36 +192,52 @@ __device__ __forceinline__ RowNorm row_norm(const float2 (&a)[8], float float2::
 #pragma unroll
     for (int o = T / 2; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
   }
-  // times 2^(127 - e); a magnitude of FF_BIG or more (its row is not transformed) as it comes
-  const float s = __uint_as_float((254u - min(top_exponent(top), 253u)) << 23);
+  const unsigned e = max(top >> 23, 1u);
+  const float s = __uint_as_float((254u - min(e, 253u)) << 23);  // the largest times s is in [1, 2)
   float q = 0.0f;
+  if (e - 80u < 94u) {  // the squares and s squared are in range
 #pragma unroll
-  for (int j = 0; j < 8; j++) q = fmaf(a[j].*row * s, a[j].*row * s, q);
-  unsigned sum = (unsigned)(q * 524288.0f);
-  if constexpr (T >= 32) {
-    sum = __reduce_add_sync(0xffffffffu, sum);
+    for (int j = 0; j < 8; j++) q = fmaf(a[j].*row, a[j].*row, q);
+    q *= s * s;
   } else {
 #pragma unroll
-    for (int o = T / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int j = 0; j < 8; j++) q = fmaf(a[j].*row * s, a[j].*row * s, q);
   }
-  return {top, sum};
+  // at most 32 x 8 squares below 4 in units of 2^-7, and the samples, in one sum
+  const unsigned sum = reduce_add<T>(((unsigned)(q * 128.0f) << 12) + some);
+  some = sum & 0xfffu;
+  return top >= FF_BIG ? FF_OUT : e + (unsigned)(max(31 - __clz((int)sum) - 19, 0) >> 1);
 }
 
-// The norm over the warps of a transform (w at distance 2).
-template <int W>
-__device__ __forceinline__ RowNorm join_norms(const RowNorm* w) {
-  RowNorm r = {0u, 0u};
+// y[n] = sum_k x[k] h[|n - k|] over the samples that are not 0, in order of k
+// (the Toeplitz product's chain), for a thread's eight outputs.
+template <int T>
+__device__ __forceinline__ void direct_sum(const float* __restrict__ x, const float* __restrict__ taps, int nch, int t,
+                                        float2 (&a)[8], float float2::*row) {
+  float y[8];
 #pragma unroll
-  for (int i = 0; i < W; i++) r.top = max(r.top, w[2 * i].top);
+  for (int j = 0; j < 8; j++) y[j] = 0.0f;
+  auto add = [&](int k, float xk) {
 #pragma unroll
-  for (int i = 0; i < W; i++)
-    r.sum += w[2 * i].sum >> min(2u * (top_exponent(r.top) - top_exponent(w[2 * i].top)), 31u);
-  return r;
-}
-
-// Biased exponent of the power of two that the norm is divided by: the norm lands in [1/2, 4).
-__device__ __forceinline__ unsigned norm_exponent(const RowNorm& r) {
-  return top_exponent(r.top) + (unsigned)(max(31 - __clz((int)r.sum) - 19, 0) >> 1);
+    for (int j = 0; j < 8; j++) y[j] = fmaf(xk, __ldg(taps + abs(min(j * T + t, nch - 1) - k)), y[j]);
+  };
+  if constexpr (T >= 32) {  // a warp's threads are all of the same transform
+    const int lane = t % 32;
+    for (int k0 = 0; k0 < nch; k0 += 32) {
+      const float xv = k0 + lane < nch ? __ldg(x + k0 + lane) : 0.0f;
+      for (unsigned m = __ballot_sync(0xffffffffu, xv != 0.0f); m; m &= m - 1u) {
+        const int b = __ffs((int)m) - 1;
+        add(k0 + b, __shfl_sync(0xffffffffu, xv, b));
+      }
+    }
+  } else {
+    for (int k = 0; k < nch; k++) {
+      const float xk = __ldg(x + k);
+      if (xk != 0.0f) add(k, xk);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; j++) a[j].*row = y[j];
 }
 
 // Rows of X [V][nr][nch] -> Y, rows as they are or (TR) in the backprojection
@@ -231,7 +257,7 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
   static_assert(T == R2 * R3, "N = 16 R2 R3");
   extern __shared__ float sm_fft[];
   __shared__ float2 s_tw2[R2 * R3];       // twiddles of pass 2, [k2][n3]
-  __shared__ RowNorm s_norm[2][NW][2];    // of the pair's rows by warp, two buffers
+  __shared__ unsigned s_row[2][2][NW];    // exponents and counts of the pair's rows by warp, two buffers
   const int tid = threadIdx.x, g = tid / T, t = tid % T;
   float* re = sm_fft + (size_t)g * 2 * PLANE;
   float* im = re + PLANE;
@@ -262,33 +288,48 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
       a[j].x = has_a && n < nch ? __ldg(xa + n) : 0.0f;
       a[j].y = has_b && n < nch ? __ldg(xb + n) : 0.0f;
     }
+    unsigned some_a = 0u, some_b = 0u;  // samples that are not 0
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      some_a += a[j].x != 0.0f ? 1u : 0u;
+      some_b += a[j].y != 0.0f ? 1u : 0u;
+    }
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const int n = j * T + t - 1;
       a[j].x -= has_a && n >= 0 && n < nch ? __ldg(xa + n) : 0.0f;
       a[j].y -= has_b && n >= 0 && n < nch ? __ldg(xb + n) : 0.0f;
     }
-    RowNorm na = row_norm<T>(a, &float2::x), nb = row_norm<T>(a, &float2::y);
+    unsigned exps = row_exponent<T>(a, &float2::x, some_a);  // row a's + 2^16 row b's, as the counts
+    exps |= row_exponent<T>(a, &float2::y, some_b) << 16;
+    unsigned some = some_a | some_b << 16;
     if constexpr (T > 32) {
       if (tid % 32 == 0) {
-        s_norm[buf][tid / 32][0] = na;
-        s_norm[buf][tid / 32][1] = nb;
+        s_row[buf][0][tid / 32] = exps;
+        s_row[buf][1][tid / 32] = some;
       }
       __syncthreads();  // also: the previous step's pass 1' has read its points
-      na = join_norms<T / 32>(&s_norm[buf][g * (T / 32)][0]);
-      nb = join_norms<T / 32>(&s_norm[buf][g * (T / 32)][1]);
+      exps = some = 0u;
+#pragma unroll
+      for (int w = 0; w < T / 32; w++) {
+        exps = __vmaxu2(exps, s_row[buf][0][g * (T / 32) + w]);
+        some += s_row[buf][1][g * (T / 32) + w];
+      }
     } else {
       __syncwarp();
     }
-    const bool bad = na.top >= FF_BIG || nb.top >= FF_BIG;  // the same for all threads of the transform
+    const unsigned ea = exps & 0xffffu, eb = exps >> 16;  // the same for all threads of the transform
+    const unsigned ca = some & 0xffffu, cb = some >> 16;
+    // rows that are summed directly
+    constexpr unsigned FEW = N > 2048 ? 128u : N > 512 ? 96u : 64u;
+    const bool sum_a = ea == FF_OUT || ca - 1u < FEW, sum_b = eb == FF_OUT || cb - 1u < FEW;
     // powers of two: row times 2^(127 - e), result times 2^(e - 127); a row of zeros gives zeros
-    const unsigned ea = norm_exponent(na), eb = norm_exponent(nb);
     const float sa = __uint_as_float((254u - ea) << 23), sb = __uint_as_float((254u - eb) << 23);
-    const float ua = na.top ? __uint_as_float(ea << 23) : 0.0f, ub = nb.top ? __uint_as_float(eb << 23) : 0.0f;
+    const float ua = ca ? __uint_as_float(ea << 23) : 0.0f, ub = cb ? __uint_as_float(eb << 23) : 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      a[j].x = bad ? 0.0f : a[j].x * sa;
-      a[j].y = bad ? 0.0f : a[j].y * sb;
+      a[j].x = sum_a ? 0.0f : a[j].x * sa;
+      a[j].y = sum_b ? 0.0f : a[j].y * sb;
     }
     {
       float2 o[8];
@@ -401,20 +442,8 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
         a[j].y *= ub;
       }
     }
-    if (bad) {
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int n = j * T + t;
-        float ya = 0.0f, yb = 0.0f;
-        if (n < nch)
-          for (int k = 0; k < nch; k++) {
-            const float h = __ldg(taps + (n > k ? n - k : k - n));
-            if (has_a) ya = fmaf(__ldg(X + m * nch + k), h, ya);
-            if (has_b) yb = fmaf(__ldg(X + (m + 1) * nch + k), h, yb);
-          }
-        a[j] = make_float2(ya, yb);
-      }
-    }
+    if (sum_a && has_a) direct_sum<T>(xa, taps, nch, t, a, &float2::x);
+    if (sum_b && has_b) direct_sum<T>(xb, taps, nch, t, a, &float2::y);
     if constexpr (TR) {
       float* y = Y + (size_t)v * nch * nrp + r0;  // nrp is a multiple of 4, r0 even
       const bool both = has_b && (reinterpret_cast<uintptr_t>(Y) & 7) == 0;  // Y may be at any float
