@@ -792,6 +792,7 @@ WFBP_API int wfbp_ctx_create(const CTGeometry* cg, const ReconConfig* rp, const 
     filter_fft_twiddles(ctx->fft_n, tw.data());
     ce = alloc_copy((void**)&ctx->d_fft_tw, tw.data(), sizeof(float2) * ctx->fft_n);
     if (!ce) ce = alloc_copy((void**)&ctx->d_fft_spec, nullptr, sizeof(float2) * ctx->fft_n);
+    if (!ce) ce = launch_filter_spectrum(ctx->d_taps, ctx->nch, ctx->fft_n, ctx->d_fft_spec, 0);
   }
   if (!ce) ce = launch_rebin_tables(ctx->d_chan_beta, ctx->d_chan_bidx, ctx->nch, cg->detector_central_col,
                                     cg->detector_pixel_size_col, cg->distance_source_to_detector, 0);
@@ -1068,18 +1069,15 @@ namespace {
 
 // FP32 filter of `rows` rows: by FFT (k_filter_fft.cu) where its transforms
 // take the channels (up to 2047), 6 to 9 times faster than the Toeplitz
-// product (k_toeplitz_f32) on scans of 96 to 1472 channels. A call computes the
-// taps' spectrum, since they may have changed (wfbp_set_taps); the later view
-// ranges of one pipelined run (spectrum = false) share it.
+// product (k_toeplitz_f32) on scans of 96 to 1472 channels. The taps' spectrum is
+// computed where the taps are set, so calls on several streams only read it.
 // The forward filter of a context whose taps are being learned (wfbp_set_taps)
 // stays a Toeplitz product: the taps' gradient is a small difference of large
 // sums (the unfiltered backprojection times the image's residual), which a
 // change of 1e-8 in the filter's gain at zero frequency moves by 1e-4; the
 // adjoint filter enters only the readings' gradient.
-int filter_rows_f32(wfbp_ctx* ctx, const float* x, float* y, long rows, bool bpl, bool fft, bool spectrum,
-                    cudaStream_t s) {
+int filter_rows_f32(wfbp_ctx* ctx, const float* x, float* y, long rows, bool bpl, bool fft, cudaStream_t s) {
   if (ctx->fft_n && fft) {
-    if (spectrum) CUDA_TRY(ctx, launch_filter_spectrum(ctx->d_taps, ctx->nch, ctx->fft_n, ctx->d_fft_spec, s));
     CUDA_TRY(ctx, launch_filter_fft(x, y, ctx->d_taps, ctx->d_fft_spec, ctx->d_fft_tw, ctx->fft_n,
                                     (int)(rows / ctx->nr), ctx->nch, ctx->nr, ctx->bpt.nrp, bpl, s));
   } else if (bpl) {
@@ -1129,7 +1127,7 @@ int do_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* scales
   }
   const float* x = (const float*)rebinned + (size_t)vb * ctx->nr * ctx->nch;
   float* y = (float*)filtered + (size_t)vb * ctx->nch * (bpl ? ctx->bpt.nrp : ctx->nr);
-  return filter_rows_f32(ctx, x, y, (long)(ve - vb) * ctx->nr, bpl, !ctx->taps_set, vb == 0, s);
+  return filter_rows_f32(ctx, x, y, (long)(ve - vb) * ctx->nr, bpl, !ctx->taps_set, s);
 }
 
 // The reference layout's rows transposed into the backprojection layout, in
@@ -1254,6 +1252,8 @@ WFBP_API int wfbp_set_taps(wfbp_ctx* ctx, const float* taps, int n, void* stream
     return fail(ctx, WFBP_ERR_UNSUPPORTED, "wfbp_set_taps: the mixed form bakes its taps into the operand planes");
   DeviceGuard g(ctx->device);
   CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_taps, taps, sizeof(float) * n, cudaMemcpyDefault, (cudaStream_t)stream));
+  if (ctx->fft_n)
+    CUDA_TRY(ctx, launch_filter_spectrum(ctx->d_taps, ctx->nch, ctx->fft_n, ctx->d_fft_spec, (cudaStream_t)stream));
   ctx->taps_set = true;
   return WFBP_OK;
 }
@@ -1335,7 +1335,7 @@ WFBP_API int wfbp_filter_adjoint(wfbp_ctx* ctx, const float* g_filtered, float* 
   if (st) return st;
   DeviceGuard g(ctx->device);
   // the Toeplitz operator h[|n - m|] is symmetric: its transpose is itself
-  return filter_rows_f32(ctx, g_filtered, g_rebinned, (long)ctx->V * ctx->nr, false, true, true, (cudaStream_t)stream);
+  return filter_rows_f32(ctx, g_filtered, g_rebinned, (long)ctx->V * ctx->nr, false, true, (cudaStream_t)stream);
 }
 
 WFBP_API int wfbp_rebin_adjoint(wfbp_ctx* ctx, const float* g_rebinned, float* g_raw, void* stream) {

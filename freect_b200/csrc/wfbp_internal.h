@@ -243,7 +243,7 @@ struct wfbp_ctx {
   // FP32 form's FFT filter (fft_n = 0: more channels than its largest transform takes)
   int fft_n = 0;                    // transform length > 2 nch
   float2* d_fft_tw = nullptr;       // [fft_n] exp(-2 pi i j / fft_n)
-  float2* d_fft_spec = nullptr;     // [fft_n] spectrum of the taps' running sums / fft_n, written by each filter call
+  float2* d_fft_spec = nullptr;     // [fft_n] spectrum of the taps' running sums / fft_n, written with the taps
   bool taps_set = false;            // wfbp_set_taps was called: the forward filter stays the Toeplitz product
 
   // TMA-staged backprojection (backprojection layout [V][nch][nrp])
