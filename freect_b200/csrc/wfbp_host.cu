@@ -989,6 +989,22 @@ WFBP_API int wfbp_selftest_bounded_wait(wfbp_ctx* ctx, int limit_ms, void* strea
   return WFBP_OK;
 }
 
+WFBP_API int wfbp_selftest_adjoint_table(wfbp_ctx* ctx, size_t limit_bytes, size_t free_bytes, int* angles) {
+  if (!ctx) return WFBP_ERR_INVALID_ARG;
+  DeviceGuard g(ctx->device);
+  if (angles) {
+    *angles = ctx->d_adj_scale ? ctx->adj_angles : 0;
+    return WFBP_OK;
+  }
+  free_dev(ctx->d_adj_scale);
+  free_dev(ctx->d_adj_gvt);
+  ctx->adj_scale_valid = false;
+  ctx->adj_angles = ctx->adj_asked = 0;
+  ctx->adj_limit = limit_bytes ? limit_bytes : kAdjointTableBytes;
+  ctx->adj_free = free_bytes;
+  return WFBP_OK;
+}
+
 WFBP_API int wfbp_get_geometry(const wfbp_ctx* ctx, CTGeometry* cg, GPUPrecompute* gp) {
   if (!ctx) return WFBP_ERR_INVALID_ARG;
   if (cg) *cg = ctx->cg;
@@ -1130,6 +1146,14 @@ int do_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* scales
   return filter_rows_f32(ctx, x, y, (long)(ve - vb) * ctx->nr, bpl, !ctx->taps_set, s);
 }
 
+// Captured work must not allocate; a stream that cannot tell counts as captured.
+bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 // The reference layout's rows transposed into the backprojection layout, in
 // memory of the context's pool in stream order (calls on several streams each
 // have their own; the pool keeps what it has until the context ends), and the
@@ -1140,11 +1164,7 @@ int do_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* scales
 bool backproject_refq(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol, const BPParams& p,
                       unsigned long long* update_count, cudaStream_t s, cudaError_t* e) {
   *e = cudaSuccess;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (!ctx->refq_ok || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return false;
-  }
+  if (!ctx->refq_ok || is_capturing(s)) return false;
   if (!ctx->refq_pool) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
@@ -1234,7 +1254,33 @@ WFBP_API int wfbp_thicken(wfbp_ctx* ctx, const float* vn, float* vol, void* stre
 // ---------------------------------------------------------------------------
 
 namespace {
-constexpr size_t kAdjointTableBytes = size_t(6) << 30;  // backprojection adjoint scale table limit
+// The adjoint's table for `most` half-turn angles of per_angle weights, or for
+// half as many as long as the memory does not suffice; none if not for one. What
+// was got is kept until the sizes change: no call repeats a failed allocation
+// that left a table.
+void alloc_adjoint_table(wfbp_ctx* ctx, size_t per_angle, int most) {
+  free_dev(ctx->d_adj_scale);
+  free_dev(ctx->d_adj_gvt);
+  ctx->adj_scale_valid = false;
+  ctx->adj_per_angle = per_angle;
+  ctx->adj_asked = most;
+  ctx->adj_angles = 0;
+  auto get = [&](float** d, size_t n) {
+    if (ctx->adj_free && n * sizeof(float) > ctx->adj_free) return false;
+    if (cudaMalloc(d, n * sizeof(float)) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+  };
+  if (!get(&ctx->d_adj_gvt, per_angle)) return;
+  for (int a = most;; a = (a + 1) / 2) {
+    if (get(&ctx->d_adj_scale, per_angle * a)) {
+      ctx->adj_angles = a;
+      return;
+    }
+    if (a == 1) break;
+  }
+  free_dev(ctx->d_adj_gvt);
+}
 
 int require_fp32_views(wfbp_ctx* ctx, const char* what) {
   if (!ctx->views_set) return fail(ctx, WFBP_ERR_STATE, std::string(what) + ": wfbp_set_views not called");
@@ -1289,42 +1335,30 @@ WFBP_API int wfbp_backproject_adjoint(wfbp_ctx* ctx, const float* g_native, floa
   for (int i = 0; i < ctx->nz && dzs != 0.0f; i++)
     if (fabsf(ctx->z_native[i] - (z0 + (float)i * dzs)) > 1e-3f * fabsf(dzs)) dzs = 0.0f;
   // The per-(voxel, theta~) scale table: whole when it fits in 6 GB (kept until
-  // the views or slices change), else for as many half-turn angles as fit at a
-  // time, refilled in every call. A refilled table costs a weight sum per
-  // (voxel, angle, slice) and a pass over it, the gather without a table a sum
-  // per (voxel, view, slice) with all its views' geometry (64 rows, 256 x 256 x
-  // 64: 8.5 against 270 ms), so that form is left to memory too small for one
-  // angle's weights.
+  // the views or slices change), else for as many half-turn angles as fit, there
+  // and in the device's free memory, refilled in every call. A refilled table
+  // costs a weight sum per (voxel, angle, slice) and a pass over it, the gather
+  // without a table a sum per (voxel, view, slice) with all its views' geometry
+  // (64 rows, 256 x 256 x 64: 8.5 against 270 ms), so that form is left to memory
+  // too small for one angle's weights, and to a captured call without a table yet
+  // (nothing may be allocated in it).
   const size_t per_angle = (size_t)ctx->nz * ctx->nx * ctx->ny;
-  int angles = (int)std::min<size_t>(ctx->P2, kAdjointTableBytes / sizeof(float) / per_angle);
+  const bool want_table = ctx->ext.adjoint_scale_table == 0 && bp_adjoint_table_ok(p, ctx->bp_nv_max);
+  const int most = want_table ? (int)std::min<size_t>(ctx->P2, ctx->adj_limit / sizeof(float) / per_angle) : 0;
+  const bool capturing = is_capturing((cudaStream_t)stream);
+  if (most > 0 && !capturing && (!ctx->d_adj_scale || per_angle != ctx->adj_per_angle || most > ctx->adj_asked))
+    alloc_adjoint_table(ctx, per_angle, most);
+  int angles = per_angle == ctx->adj_per_angle ? std::min(most, ctx->adj_angles) : 0;
   if (angles > 0 && angles < ctx->P2) {
     const int groups = (ctx->P2 + angles - 1) / angles;  // equal groups
     angles = (ctx->P2 + groups - 1) / groups;
   }
-  const size_t n = per_angle * angles;
-  const bool want_table =
-      ctx->ext.adjoint_scale_table == 0 && angles > 0 && bp_adjoint_table_ok(p, ctx->bp_nv_max);
-  if (want_table && (n > ctx->adj_scale_n || per_angle > ctx->adj_gvt_n)) {
-    free_dev(ctx->d_adj_scale);
-    free_dev(ctx->d_adj_gvt);
-    ctx->adj_scale_valid = false;
-    if (cudaMalloc(&ctx->d_adj_scale, n * sizeof(float)) == cudaSuccess &&
-        cudaMalloc(&ctx->d_adj_gvt, per_angle * sizeof(float)) == cudaSuccess) {
-      ctx->adj_scale_n = n;
-      ctx->adj_gvt_n = per_angle;
-    } else {
-      cudaGetLastError();  // too large for the free memory: recompute the sums instead
-      free_dev(ctx->d_adj_scale);
-      free_dev(ctx->d_adj_gvt);
-      ctx->adj_scale_n = ctx->adj_gvt_n = 0;
-    }
-  }
-  float* table = want_table && ctx->d_adj_scale && ctx->d_adj_gvt ? ctx->d_adj_scale : nullptr;
+  float* table = angles > 0 ? ctx->d_adj_scale : nullptr;
   const bool whole = angles == ctx->P2;
   CUDA_TRY(ctx, launch_bp_adjoint(g_native, g_filtered, ctx->d_view_sc, ctx->d_view_z, ctx->d_z_native, p, z0, dzs,
                                   table, angles, table && !(whole && ctx->adj_scale_valid), ctx->d_adj_gvt,
                                   ctx->bp_reach, ctx->bp_nv_max, (cudaStream_t)stream));
-  if (table) ctx->adj_scale_valid = whole;
+  if (table && !capturing) ctx->adj_scale_valid = whole;  // a captured fill runs with its graph
   return WFBP_OK;
 }
 

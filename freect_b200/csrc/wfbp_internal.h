@@ -170,6 +170,8 @@ struct RebinParams {
 // consecutive views per thread.
 constexpr int RV_CW = 128, RV_NY = 4;
 
+constexpr size_t kAdjointTableBytes = size_t(6) << 30;  // backprojection adjoint scale table limit
+
 struct wfbp_ctx {
   CTGeometry cg;                    // geometry of the views the stages work on (effective one with FFS)
   CTGeometry cg_read;               // geometry of the raw readings (== cg without FFS)
@@ -226,9 +228,10 @@ struct wfbp_ctx {
   float* d_tg_partial = nullptr;    // per-CTA partial tap gradients
   size_t tg_partial_n = 0;
   float* d_adj_scale = nullptr;     // backprojection adjoint: per-(voxel, theta~) weight dtheta / sum_k W_k
-  size_t adj_scale_n = 0;
   float* d_adj_gvt = nullptr;       // backprojection adjoint: gradient as [nz][nx][ny]
-  size_t adj_gvt_n = 0;
+  size_t adj_per_angle = 0;         // weights of one half-turn angle in the table
+  int adj_angles = 0, adj_asked = 0;  // angles it holds; angles that were asked for
+  size_t adj_limit = kAdjointTableBytes, adj_free = 0;  // most bytes of the table; test hook: larger allocations fail
   bool adj_scale_valid = false;     // the table matches the current views and slices
 
   // mixed precision: Toeplitz operand planes for the tensor-core filter

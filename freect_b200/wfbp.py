@@ -47,6 +47,7 @@ _PROTOS = {
     "wfbp_last_error": (C.c_char_p, [_VP]),
     "wfbp_check_device_status": (C.c_int, [_VP]),
     "wfbp_selftest_bounded_wait": (C.c_int, [_VP, C.c_int, _VP]),
+    "wfbp_selftest_adjoint_table": (C.c_int, [_VP, C.c_size_t, C.c_size_t, C.POINTER(C.c_int)]),
     "wfbp_status_string": (C.c_char_p, [C.c_int]),
     "wfbp_rebin": (C.c_int, [_VP, _VP, _VP, _VP]),
     "wfbp_filter": (C.c_int, [_VP, _VP, _VP, _VP, _VP]),
@@ -252,6 +253,18 @@ class Context:
         """Runs a wait that can never complete, bounded to limit_ms."""
         _check(self._lib.wfbp_selftest_bounded_wait(self._h, int(limit_ms), _stream(stream)),
                "wfbp_selftest_bounded_wait", self._h)
+
+    def selftest_adjoint_table(self, limit_bytes=0, free_bytes=0):
+        """Releases the adjoint's weight table and bounds the next one (wfbp_selftest_adjoint_table)."""
+        _check(self._lib.wfbp_selftest_adjoint_table(self._h, int(limit_bytes), int(free_bytes), None),
+               "wfbp_selftest_adjoint_table", self._h)
+
+    def selftest_adjoint_angles(self):
+        """Half-turn angles that the adjoint's weight table holds."""
+        n = C.c_int()
+        _check(self._lib.wfbp_selftest_adjoint_table(self._h, 0, 0, C.byref(n)), "wfbp_selftest_adjoint_table",
+               self._h)
+        return n.value
 
     @property
     def handle(self):

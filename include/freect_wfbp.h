@@ -207,7 +207,9 @@ typedef struct wfbp_ext {
   int adjoint_scale_table;    /* 0: the backprojection adjoint keeps a per-(voxel, half-turn angle)
                                  weight table dtheta / sum_k W_k when it fits in 6 GB, computed on
                                  the first adjoint call after the views or slices change; a larger
-                                 one is computed in every call, as many angles at a time as fit;
+                                 one, or one the free memory does not hold, is computed in every
+                                 call, as many angles at a time as fit; nothing is allocated in a
+                                 captured call (it uses the table that is there);
                                  -1: never (the adjoint recomputes the weight sums) */
   int reserved[5];
 } wfbp_ext;
@@ -361,6 +363,12 @@ int wfbp_check_device_status(wfbp_ctx* ctx);
  * WFBP_ERR_TIMEOUT and the context stays usable. Every production wait
  * (TMA rings, tensor-core pipeline) is bounded the same way (4 s). */
 int wfbp_selftest_bounded_wait(wfbp_ctx* ctx, int limit_ms, void* stream);
+
+/* Memory self-test of the backprojection adjoint's weight table: with angles ==
+ * NULL the table is released and may take limit_bytes from the next adjoint
+ * call on (0: 6 GB), and its allocations above free_bytes are taken as failed
+ * (0: none is); else *angles receives the half-turn angles it holds now. */
+int wfbp_selftest_adjoint_table(wfbp_ctx* ctx, size_t limit_bytes, size_t free_bytes, int* angles);
 
 /* Last error message of this context (never NULL). */
 const char* wfbp_last_error(const wfbp_ctx* ctx);
