@@ -109,7 +109,8 @@ class Ext(C.Structure):
         ("bp_slab", C.c_int),
         ("filtered_layout", C.c_int),
         ("adjoint_scale_table", C.c_int),
-        ("reserved", C.c_int * 5),
+        ("backproject_scratch", C.c_int),
+        ("reserved", C.c_int * 4),
     ]
 
 

@@ -1154,33 +1154,43 @@ bool is_capturing(cudaStream_t s) {
   return true;
 }
 
+// The context's stream-ordered pool, made at its first use (by any thread).
+// It keeps at most kRefqKeepBytes between calls; what a larger scan took goes
+// back to the device when the work that used it is next waited for.
+cudaMemPool_t refq_pool(wfbp_ctx* ctx) {
+  constexpr cuuint64_t kRefqKeepBytes = 256u << 20;
+  std::lock_guard<std::mutex> lock(ctx->refq_mutex);
+  if (ctx->refq_pool) return ctx->refq_pool;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = ctx->device;
+  cudaMemPool_t pool = nullptr;
+  cuuint64_t keep = kRefqKeepBytes;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    if (pool) cudaMemPoolDestroy(pool);
+    cudaGetLastError();
+    return nullptr;
+  }
+  return ctx->refq_pool = pool;
+}
+
 // The reference layout's rows transposed into the backprojection layout, in
 // memory of the context's pool in stream order (calls on several streams each
-// have their own; the pool keeps what it has until the context ends), and the
-// TMA-staged kernel on them with k_bp's arithmetic: 16 rows, 256 x 256 x 26
-// FP32 11.4 ms by k_bp's gathers from L2, 6.4 here, 0.06 of them the
-// transpose. False: not done, k_bp has to (no launch fits, no memory, or the
-// stream is being captured: a graph would own the memory).
+// have their own), and the TMA-staged kernel on them with k_bp's arithmetic: 16
+// rows, 256 x 256 x 26 FP32 11.4 ms by k_bp's gathers from L2, 6.4 here, 0.06 of
+// them the transpose. False: not done, k_bp has to (the context refuses it, no
+// launch fits, no memory, or the stream is being captured: a graph would own the
+// memory).
 bool backproject_refq(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol, const BPParams& p,
                       unsigned long long* update_count, cudaStream_t s, cudaError_t* e) {
   *e = cudaSuccess;
-  if (!ctx->refq_ok || is_capturing(s)) return false;
-  if (!ctx->refq_pool) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = ctx->device;
-    cuuint64_t keep = ~0ull;
-    if (cudaMemPoolCreate(&ctx->refq_pool, &props) != cudaSuccess ||
-        cudaMemPoolSetAttribute(ctx->refq_pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-      if (ctx->refq_pool) cudaMemPoolDestroy(ctx->refq_pool);
-      ctx->refq_pool = nullptr;
-      cudaGetLastError();
-      return false;
-    }
-  }
+  if (ctx->ext.backproject_scratch == -1 || !ctx->refq_ok || is_capturing(s)) return false;
+  const cudaMemPool_t pool = refq_pool(ctx);
+  if (!pool) return false;
   void* d = nullptr;
-  if (cudaMallocFromPoolAsync(&d, sizeof(float) * (size_t)ctx->V * ctx->nch * ctx->refq.nrp, ctx->refq_pool, s) !=
+  if (cudaMallocFromPoolAsync(&d, sizeof(float) * (size_t)ctx->V * ctx->nch * ctx->refq.nrp, pool, s) !=
       cudaSuccess) {
     cudaGetLastError();
     return false;

@@ -7,6 +7,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -264,6 +265,7 @@ struct wfbp_ctx {
   bool refq_ok = false;
   BPTile refq;
   cudaMemPool_t refq_pool = nullptr;
+  std::mutex refq_mutex;            // guards the pool's creation
 
   // context-owned scratch for wfbp_run / wfbp_run_host
   void* s_rebinned = nullptr;

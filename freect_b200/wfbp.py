@@ -195,7 +195,8 @@ def recon_kernel_filter(recon_kernel):
 
 
 def make_ext(precision=T.PRECISION_FP32, filter_window=T.FILTER_REFERENCE, filter_c=1.0, filter_a=1.0,
-             user_taps=None, tex_weights=0, bp_slab=0, filtered_layout=T.LAYOUT_REFERENCE, adjoint_scale_table=0):
+             user_taps=None, tex_weights=0, bp_slab=0, filtered_layout=T.LAYOUT_REFERENCE, adjoint_scale_table=0,
+             backproject_scratch=0):
     e = T.Ext()
     e.version = T.EXT_VERSION
     e.precision = precision
@@ -206,6 +207,7 @@ def make_ext(precision=T.PRECISION_FP32, filter_window=T.FILTER_REFERENCE, filte
     e.bp_slab = bp_slab
     e.filtered_layout = filtered_layout
     e.adjoint_scale_table = adjoint_scale_table
+    e.backproject_scratch = backproject_scratch
     if user_taps is not None:
         arr = np.ascontiguousarray(user_taps, dtype=np.float32)
         e._taps_keepalive = arr

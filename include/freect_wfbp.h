@@ -211,7 +211,9 @@ typedef struct wfbp_ext {
                                  call, as many angles at a time as fit; nothing is allocated in a
                                  captured call (it uses the table that is there);
                                  -1: never (the adjoint recomputes the weight sums) */
-  int reserved[5];
+  int backproject_scratch;    /* -1: wfbp_backproject takes no device memory (reference layout:
+                                 the gather kernel, about half as fast); otherwise see there */
+  int reserved[4];
 } wfbp_ext;
 
 /* Sizes of every stage buffer a context expects (bytes unless noted). */
@@ -397,7 +399,14 @@ int wfbp_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* row_
 /* ReconstructionMachine::Backproject (ReconstructionMachine.cu:308-385,
  * backproject_kernel cuda_kernels.cuh:198-287). volume_native: FP32
  * [nz_native][ny][nx], overwritten. update_count: optional device uint64
- * that receives the number of contributing voxel-view updates (adds to it). */
+ * that receives the number of contributing voxel-view updates (adds to it).
+ * Reference layout: unless the context refuses (wfbp_ext.backproject_scratch =
+ * -1), the rows are first copied, transposed, to device memory of V * n_channels
+ * * (n_rows rounded up to 4) floats that the call takes from a pool of the
+ * context in stream order. The pool keeps up to 256 MiB between calls (until
+ * wfbp_ctx_destroy), more goes back to the device at the next synchronisation.
+ * Where that memory is not to be had, and in a captured call, the gather kernel
+ * runs on the caller's rows: the same samples, the sums' last bits may differ. */
 int wfbp_backproject(wfbp_ctx* ctx, const void* filtered, const float* row_scales,
                      float* volume_native, unsigned long long* update_count, void* stream);
 
