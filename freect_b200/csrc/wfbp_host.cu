@@ -280,10 +280,6 @@ void mixed_scale_ptrs(const wfbp_ctx* ctx, P rebinned, float** row_sc, float** v
   *op_sc = reinterpret_cast<float*>(b + o_view + al256((size_t)ctx->V * sizeof(float)));
 }
 
-// Sizes the TMA-staged backprojection for this geometry: the column tile, the
-// channel window each view needs for it, and the most views of one theta~ that
-// can reach a slab. Returns false if no configuration fits in shared
-// memory (the generic kernel is used then).
 // Slab-level view reach and the most views of one theta~ that can reach a
 // slab of 16 or 32 slices; both depend only on the geometry and the table
 // positions.
@@ -294,6 +290,7 @@ void bp_reach(wfbp_ctx* ctx, const std::vector<float>& table) {
   // |z - z_j| <= |A| + l_hat tan for any valid (voxel, view); tighter than z_rot
   const double cone = (R + rmax) * tanc + (ctx->cg.z_rot / (2 * M_PI)) * asin(std::min(1.0, rmax / R));
   const double reach = std::min((double)ctx->cg.z_rot, cone) + 1e-3 * (1.0 + fabs(ctx->cg.z_rot));
+  const int order = bp_table_order(table.data(), ctx->K * ctx->P2);
   for (int slab = 16; slab <= 32; slab += 16) {
     int nv_max = 1;
     for (int s0 = 0; s0 < ctx->nz; s0 += slab) {
@@ -303,14 +300,7 @@ void bp_reach(wfbp_ctx* ctx, const std::vector<float>& table) {
         zmx = std::max(zmx, ctx->z_native[i]);
       }
       const float lo = zmn - (float)reach, hi = zmx + (float)reach;
-      for (int t = 0; t < ctx->P2; t++) {
-        int n = 0;
-        for (int k = 0; k < ctx->K; k++) {
-          const float zt = table[t + k * ctx->P2];
-          if (!(zt < lo || zt > hi)) n++;
-        }
-        nv_max = std::max(nv_max, n);
-      }
+      nv_max = std::max(nv_max, bp_most_views(table.data(), order, ctx->P2, ctx->K, lo, hi));
     }
     (slab == 16 ? ctx->bp_nv_max16 : ctx->bp_nv_max) = nv_max;
   }

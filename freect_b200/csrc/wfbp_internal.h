@@ -7,6 +7,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -81,6 +82,44 @@ inline int bp_theta_chunks(int nx, int ny, int nz, int P2, size_t window_bytes) 
 // which only such a launch has) when there are several.
 __host__ __device__ constexpr bool bp_exchanges(int nc) { return nc > 1; }
 __host__ __device__ inline int bp_chunk_begin(int chunk, int nc, int P2) { return (int)((long)P2 * chunk / nc); }
+
+// 1: the n table positions never fall, -1: they never rise (a table that stands
+// still counts as 1), 0: neither.
+inline int bp_table_order(const float* table, int n) {
+  bool up = true, down = true;
+  for (int j = 1; j < n; j++) {
+    up = up && table[j] >= table[j - 1];
+    down = down && table[j] <= table[j - 1];
+  }
+  return up ? 1 : down ? -1 : 0;
+}
+// Most views of one half-turn angle (views t, t + P2, ..., K of them) with a table
+// position in [lo, hi]. In an ordered table they are a run of consecutive views,
+// of which an angle has every P2-th: two searches instead of a walk over all views
+// (64 rows, 9840 views, 45 slabs: 0.4 ms of a context's preparation).
+inline int bp_most_views(const float* table, int order, int P2, int K, float lo, float hi) {
+  if (order) {
+    const float *end = table + (size_t)K * P2, *a, *b;
+    if (order > 0) {
+      a = std::partition_point(table, end, [&](float z) { return z < lo; });
+      b = std::partition_point(a, end, [&](float z) { return z <= hi; });
+    } else {
+      a = std::partition_point(table, end, [&](float z) { return z > hi; });
+      b = std::partition_point(a, end, [&](float z) { return z >= lo; });
+    }
+    return (int)((b - a + P2 - 1) / P2);
+  }
+  int most = 0;
+  for (int t = 0; t < P2; t++) {
+    int n = 0;
+    for (int k = 0; k < K; k++) {
+      const float z = table[t + (size_t)k * P2];
+      if (!(z < lo || z > hi)) n++;
+    }
+    most = std::max(most, n);
+  }
+  return most;
+}
 
 // Bits of the device-side error word besides WFBP_ERR_TIMEOUT (which a
 // bounded wait that gave up stores whole): conditions the host's sizing rules
