@@ -469,6 +469,14 @@ k_filter_fft(const float* __restrict__ X, float* __restrict__ Y, const float* __
   }
 }
 
+// tw[j] = exp(-2 pi i j / N), rounded from FP64.
+__global__ void __launch_bounds__(256) k_filter_twiddles(int N, float2* __restrict__ tw) {
+  const int j = blockIdx.x * 256 + threadIdx.x;
+  double s, c;
+  sincospi(-2.0 * (double)j / (double)N, &s, &c);
+  tw[j] = make_float2((float)c, (float)s);
+}
+
 // A[f] / N, the spectrum of the running sums a of the symmetric taps. a's
 // differences are h inside the window [-nch, nch) and -S / 2 at both its ends
 // (S = H[0], the sum of all taps), so with w = 2 pi f / N and
@@ -555,11 +563,9 @@ int filter_fft_size(int nch) {
   return 0;
 }
 
-void filter_fft_twiddles(int N, float2* tw) {
-  for (int j = 0; j < N; j++) {
-    const double a = -2.0 * M_PI * (double)j / (double)N;
-    tw[j] = make_float2((float)cos(a), (float)sin(a));
-  }
+cudaError_t launch_filter_twiddles(int N, float2* tw, cudaStream_t s) {
+  k_filter_twiddles<<<(unsigned)(N / 256), 256, 0, s>>>(N, tw);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_filter_spectrum(const float* d_taps, int nch, int N, float2* spec, cudaStream_t s) {

@@ -172,7 +172,6 @@ void release(wfbp_ctx* ctx) {
   free_dev(ctx->d_fuse_tab);
   free_dev(ctx->d_bplanes);
   free_dev(ctx->d_fft_tw);
-  free_dev(ctx->d_fft_spec);
   free_dev(ctx->d_err);
   free_dev(ctx->d_thickT_off);
   free_dev(ctx->d_thickT_idx);
@@ -778,10 +777,9 @@ WFBP_API int wfbp_ctx_create(const CTGeometry* cg, const ReconConfig* rp, const 
     if (!ce) ce = alloc_copy((void**)&ctx->d_chan64, ch.data(), sizeof(double2) * nch);
   }
   if (!ce && e.precision == WFBP_PRECISION_FP32 && (ctx->fft_n = filter_fft_size(ctx->nch)) > 0) {
-    std::vector<float2> tw(ctx->fft_n);
-    filter_fft_twiddles(ctx->fft_n, tw.data());
-    ce = alloc_copy((void**)&ctx->d_fft_tw, tw.data(), sizeof(float2) * ctx->fft_n);
-    if (!ce) ce = alloc_copy((void**)&ctx->d_fft_spec, nullptr, sizeof(float2) * ctx->fft_n);
+    ce = alloc_copy((void**)&ctx->d_fft_tw, nullptr, sizeof(float2) * 2 * ctx->fft_n);
+    ctx->d_fft_spec = ctx->d_fft_tw ? ctx->d_fft_tw + ctx->fft_n : nullptr;
+    if (!ce) ce = launch_filter_twiddles(ctx->fft_n, ctx->d_fft_tw, 0);
     if (!ce) ce = launch_filter_spectrum(ctx->d_taps, ctx->nch, ctx->fft_n, ctx->d_fft_spec, 0);
   }
   if (!ce) ce = launch_rebin_tables(ctx->d_chan_beta, ctx->d_chan_bidx, ctx->nch, cg->detector_central_col,

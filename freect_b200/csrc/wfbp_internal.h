@@ -285,7 +285,7 @@ struct wfbp_ctx {
 
   // FP32 form's FFT filter (fft_n = 0: more channels than its largest transform takes)
   int fft_n = 0;                    // transform length > 2 nch
-  float2* d_fft_tw = nullptr;       // [fft_n] exp(-2 pi i j / fft_n)
+  float2* d_fft_tw = nullptr;       // [fft_n] exp(-2 pi i j / fft_n), and the spectrum behind them
   float2* d_fft_spec = nullptr;     // [fft_n] spectrum of the taps' running sums / fft_n, written with the taps
   bool taps_set = false;            // wfbp_set_taps was called: the forward filter stays the Toeplitz product
 
@@ -367,7 +367,7 @@ cudaError_t launch_filter_f32_tr(const float* x, float* yt, const float* d_taps,
 // FFT form of the FP32 filter (k_filter_fft.cu): transform length for nch
 // channels (0: none), its twiddles, the taps' spectrum, the filter itself
 int filter_fft_size(int nch);
-void filter_fft_twiddles(int N, float2* tw);
+cudaError_t launch_filter_twiddles(int N, float2* tw, cudaStream_t s);
 cudaError_t launch_filter_spectrum(const float* d_taps, int nch, int N, float2* spec, cudaStream_t s);
 cudaError_t launch_filter_fft(const float* x, float* y, const float* d_taps, const float2* spec, const float2* tw, int N,
                               int V, int nch, int nr, int nrp, bool transposed, cudaStream_t s);
