@@ -112,7 +112,7 @@ struct __align__(16) GeoQ {
   float2 wp;
 };
 // Record of the reference layout's form (REFQ): k_bp's own arithmetic per
-// slice, q = (((z - zt) + zr2pi asn) inv + 1) hn with the roundings that
+// sample (an angle's quotient is the other forms'), q = (((z - zt) + zr2pi asn) inv + 1) hn with the roundings that
 // kernel has, so that a sample at the edge of the detector falls the same way.
 struct __align__(16) GeoR {
   float2 inv, asn;  // 1 / (l_hat tan(cone)), asin(p_hat / R) (an invalid record: 1, -1e30)

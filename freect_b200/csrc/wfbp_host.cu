@@ -353,7 +353,9 @@ const int kBpCandidates[][5] = {
     {16, 8, 4, 8, 16},   {16, 8, 8, 8, 16},   {8, 16, 8, 8, 16}};
 
 // ext.bp_slab, when set, admits only configurations with slabs of that height
-bool slab_allowed(const wfbp_ctx* ctx, int slab) { return ctx->ext.bp_slab == 0 || ctx->ext.bp_slab == slab; }
+// (of the backprojection layout: `only` = 0 for the reference layout's launch)
+bool slab_allowed(int only, int slab) { return only == 0 || only == slab; }
+bool slab_allowed(const wfbp_ctx* ctx, int slab) { return slab_allowed(ctx->ext.bp_slab, slab); }
 
 // The launch shape a context starts with (an autotuner may set another). The
 // kernel is bound by instruction issue and hides its latencies with resident
@@ -361,7 +363,7 @@ bool slab_allowed(const wfbp_ctx* ctx, int slab) { return ctx->ext.bp_slab == 0 
 // 32-slice one, so: 8 x 16 columns / 8 warps / 16 slices where three CTAs fit an
 // SM (24 consumer warps), else 16 x 20 / 20 / 16 (20 warps in one CTA: wide view
 // windows, as a flying focal spot's), else the first candidate that fits. With
-// the mixed form's pairs and a cone of 48 slices or more the lanes' view lists
+// the mixed form's pairs and 48 detector rows or more the lanes' view lists
 // fill a 32-slice slab as well, and its geometry records serve twice the lanes:
 // 8 x 16 / 8 / 32 where two CTAs fit, else 16 x 16 / 16 / 32. Measured, ms, 16-slice
 // shape / 32-slice shape: 64 rows 512 x 512 x 96 mixed 39.4 / 38.2, FP32 39.5 /
@@ -369,16 +371,16 @@ bool slab_allowed(const wfbp_ctx* ctx, int slab) { return ctx->ext.bp_slab == 0 
 // FP32 47.4 / 47.3; 32 rows mixed 7.0 / 8.0; 20 rows mixed 15.4 / 17.3; 16 rows
 // mixed 4.64 / 5.04. 8 x 16 / 8 / 16 in two CTAs instead of 16 x 20 / 20 / 16: flying
 // focal spot FP32 70.5 against 47.4.
-bool default_bp_tile(const wfbp_ctx* ctx, bool pairs, BPTile* out) {
+bool default_bp_tile(const wfbp_ctx* ctx, bool pairs, int only, BPTile* out) {
   BPTile b;
-  if (pairs && ctx->nr >= 48 && slab_allowed(ctx, 32) && ctx->nz > 16) {
+  if (pairs && ctx->nr >= 48 && slab_allowed(only, 32) && ctx->nz > 16) {
     if (size_bp_tile(ctx, 8, 16, 8, 8, 32, &b) && 2 * (b.smem_bytes + 1024) <= 228 * 1024) {
       *out = b;
       return true;
     }
     if (size_bp_tile(ctx, 16, 16, 8, 16, 32, out)) return true;
   }
-  if (!slab_allowed(ctx, 16)) return false;
+  if (!slab_allowed(only, 16)) return false;
   if (size_bp_tile(ctx, 8, 16, 8, 8, 16, &b) && 3 * (b.smem_bytes + 1024) <= 228 * 1024) {
     *out = b;
     return true;
@@ -392,11 +394,7 @@ void choose_refq_tile(wfbp_ctx* ctx) {
   BPTile b;
   ctx->refq_ok = false;
   if (!(ctx->gp.z_rot_over_2_pi > 0.0f)) return;
-  wfbp_ext any = ctx->ext;
-  any.bp_slab = 0;  // restricts the backprojection layout's shapes only
-  std::swap(ctx->ext, any);
-  const bool fits = default_bp_tile(ctx, false, &b) || size_bp_tile(ctx, 8, 8, 4, 16, 32, &b);
-  std::swap(ctx->ext, any);
+  const bool fits = default_bp_tile(ctx, false, 0, &b) || size_bp_tile(ctx, 8, 8, 4, 16, 32, &b);
   if (!fits || !bp_refq_supported(b)) return;
   b.zc = 0;
   b.smem_bytes = (int)bp_tma_smem_bytes(b, 4);
@@ -407,7 +405,7 @@ void choose_refq_tile(wfbp_ctx* ctx) {
 bool choose_bp_tile(wfbp_ctx* ctx, const std::vector<float>& table) {
   bp_reach(ctx, table);
   choose_refq_tile(ctx);
-  if (default_bp_tile(ctx, ctx->ext.precision == WFBP_PRECISION_MIXED, &ctx->bpt)) return true;
+  if (default_bp_tile(ctx, ctx->ext.precision == WFBP_PRECISION_MIXED, ctx->ext.bp_slab, &ctx->bpt)) return true;
   for (auto& c : kBpCandidates) {
     if (!slab_allowed(ctx, c[4])) continue;
     BPTile b;
@@ -1166,9 +1164,10 @@ cudaMemPool_t refq_pool(wfbp_ctx* ctx) {
 
 // The reference layout's rows transposed into the backprojection layout, in
 // memory of the context's pool in stream order (calls on several streams each
-// have their own), and the TMA-staged kernel on them with k_bp's arithmetic: 16
-// rows, 256 x 256 x 26 FP32 11.4 ms by k_bp's gathers from L2, 6.4 here, 0.06 of
-// them the transpose. False: not done, k_bp has to (the context refuses it, no
+// have their own), and the TMA-staged kernel on them with k_bp's arithmetic (but
+// for the quotient of an angle's sums, taken through the hardware reciprocal):
+// 16 rows, 256 x 256 x 26 FP32 11.4 ms by k_bp's gathers from L2, 5.7 here, 0.06
+// of them the transpose. False: not done, k_bp has to (the context refuses it, no
 // launch fits, no memory, or the stream is being captured: a graph would own the
 // memory).
 bool backproject_refq(wfbp_ctx* ctx, const void* filtered, const float* scales, float* vol, const BPParams& p,

@@ -389,8 +389,15 @@ const char* wfbp_status_string(int status);
 int wfbp_rebin(wfbp_ctx* ctx, const float* raw, void* rebinned, void* stream);
 
 /* Stage 2 of RebinAndFilter (ReconstructionMachine.cu:262-290: R2C,
- * multiply_filter, C2R, reshape_rebin_into_final_array) as a Toeplitz
- * contraction. filtered: FP32 [V][nr][nch] (FP32) or FP16 [V][nr][nch]
+ * multiply_filter, C2R, reshape_rebin_into_final_array) as the linear
+ * convolution with the symmetric taps. FP32 with at most 2047 channels: by FFT,
+ * whose error is relative to the row's 2-norm (about 1e-7; a row of at most 64
+ * samples that are not 0 is summed directly), so that samples far outside the
+ * object, thousands of times smaller than the row's largest, are less exact
+ * relative to themselves than a direct sum's. More channels, and every forward
+ * call of a context once wfbp_set_taps was called (the taps' gradient is a small
+ * difference of large sums): a Toeplitz contraction, 6 to 9 times slower. MIXED: a
+ * Toeplitz contraction on the tensor cores. filtered: FP32 [V][nr][nch] (FP32) or FP16 [V][nr][nch]
  * plus row_scales FP32 [V][nr] (MIXED; row_scales may be NULL for FP32), in
  * the reference layout; in the backprojection layout see wfbp_layout. */
 int wfbp_filter(wfbp_ctx* ctx, const void* rebinned, void* filtered, float* row_scales,
@@ -506,7 +513,9 @@ const char* wfbp_batch_last_error(const wfbp_batch* batch);
 /* Overwrites taps h[0..n-1] of the context's symmetric half taps (device or
  * host pointer, stream-ordered copy) -- the learnable part of the filter.
  * The taps start as generate_filter's (ReconstructionMachine.cu:478-513)
- * or the ext's window; wfbp_get_taps reads all n_channels of them. */
+ * or the ext's window; wfbp_get_taps reads all n_channels of them. From the
+ * first call on the context's forward filter is a Toeplitz contraction (see
+ * wfbp_filter). */
 int wfbp_set_taps(wfbp_ctx* ctx, const float* taps, int n, void* stream);
 int wfbp_get_taps(wfbp_ctx* ctx, float* taps, void* stream);
 
@@ -520,7 +529,8 @@ int wfbp_thicken_adjoint(wfbp_ctx* ctx, const float* g_volume, float* g_native, 
 int wfbp_backproject_adjoint(wfbp_ctx* ctx, const float* g_native, float* g_filtered, void* stream);
 
 /* Transpose of wfbp_filter (FP32): the Toeplitz operator is symmetric, so
- * this filters g_filtered [V][nr][nch] with the same taps. */
+ * this filters g_filtered [V][nr][nch] with the same taps, with up to 2047
+ * channels by FFT (see wfbp_filter for its error). */
 int wfbp_filter_adjoint(wfbp_ctx* ctx, const float* g_filtered, float* g_rebinned, void* stream);
 
 /* Transpose of wfbp_rebin: g_rebinned [V][nr][nch] -> g_raw
