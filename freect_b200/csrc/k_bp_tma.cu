@@ -304,6 +304,10 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
     const float ya = ycoord(iy0), yb = ycoord(min(iy0 + bt.ty - 1, p.ny - 1));
     const uint32_t view_bytes = (uint32_t)(bt.W * bt.nrp * sizeof(T));
     const unsigned below = (1u << lane) - 1u;
+    // no lists where a slice range can be NaN: the tile has a corner beyond the
+    // source's orbit (|p_hat| >= R for some angle)
+    const bool lists = bt.nv_max <= BP_LIST_VIEWS &&
+                       fmaxf(xa * xa, xb * xb) + fmaxf(ya * ya, yb * yb) < 0.999f * p.R2;
     int issued_upto = 0;
     bool failed = false;
     for (int t = tb; t < te; t++) {
@@ -338,9 +342,8 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
             const float t1 = xa * sc.y + ya * sc.x, t2 = xa * sc.y + yb * sc.x;
             const float t3 = xb * sc.y + ya * sc.x, t4 = xb * sc.y + yb * sc.x;
             const float lhi = sqrtf(p.R2) - fminf(fminf(t1, t2), fminf(t3, t4));
-            // (a corner beyond the source's orbit: no voxel of the field has |p_hat| >= R, the clamp keeps the bound)
-            const float amin = p.zr2pi * asinf(fmaxf(p.rR * pmin, -1.0f)),
-                        amax = p.zr2pi * asinf(fminf(p.rR * pmax, 1.0f));
+            // (a bound is NaN at a corner beyond the source's orbit: then it excludes no view)
+            const float amin = p.zr2pi * asinf(p.rR * pmin), amax = p.zr2pi * asinf(p.rR * pmax);
             const float eps = 1e-3f * (1.0f + fabsf(zt));
             wlo = zt - amax - lhi * p.tanc - eps;
             whi = zt - amin + lhi * p.tanc + eps;
@@ -378,7 +381,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         // lane = slice: the views, in order, whose slice range holds it
         uint32_t list = 0u;
         int n = 0;
-        if (nv > 1 && bt.nv_max <= BP_LIST_VIEWS)
+        if (nv > 1 && lists)
           for (int v = 0; v < nv; v++) {
             const float2 w = vwin[v];
             if (zl >= w.x && zl <= w.y) {
@@ -392,7 +395,7 @@ __device__ __forceinline__ int bp_tile(const CUtensorMap* map, float* __restrict
         // Steps over lists cost more each (lanes on two views' samples meet in
         // the banks, more so with FP32 rows' eight loads per pair): every view
         // for every lane unless they save enough.
-        const bool pays = nv > 1 && bt.nv_max <= BP_LIST_VIEWS && most <= 8 &&
+        const bool pays = nv > 1 && lists && most <= 8 &&
                           (HALF ? 6 * most < 5 * nv : 3 * most <= 2 * nv);
         vlist[s * 32 + lane] = pays ? list : 0x76543210u;
         if (lane == 0) nvs[2 + s] = pays ? most : nv;
