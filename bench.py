@@ -710,7 +710,8 @@ def stage_rooflines(form, ctx, d, updates, stage, clk):
     rebin: HBM, raw frames read once + rebinned output written once.
     filter: tensor pipe (mixed: 3 split-FP16 products of 2 (V nr) nch^2
     FLOP each, against the sustained cuBLAS BF16 rate, the same tensor rate
-    as FP16); FP32 form: HBM (FFT, rows read and written once), beyond 2047
+    as FP16); FP32 form: the FFT is bound by shared-memory wavefronts and issue,
+    its rate is given against HBM (rows read and written once); beyond 2047
     channels FP32 FFMA (2 (V nr) nch^2 FLOP against 148 SMs x 128 lanes x 2 x
     clock)."""
     hbm, bf16, bf16_sus, peak_src = load_peaks()
@@ -752,9 +753,11 @@ def stage_rooflines(form, ctx, d, updates, stage, clk):
                 "note": "3 split-FP16 products (hi*hi, hi*lo, lo*hi) of 2 M K N, M = views x rows, K = N = "
                         "channels, against the sustained cuBLAS BF16 rate (FP16 runs at the same tensor rate)"}
     elif d.n_channels < 2048:  # k_filter_fft
-        filt = {"bound": "hbm", "kernel": "filter_fft", "achieved": samples * 8 / t_f / 1e9, "peak": hbm, "unit": "GB/s",
+        filt = {"bound": "shared memory and issue", "kernel": "filter_fft", "achieved": samples * 8 / t_f / 1e9, "peak": hbm, "unit": "GB/s",
                 "frac": samples * 8 / t_f / 1e9 / hbm, "algorithmic_bytes": samples * 8,
-                "note": "FP32 FFT filter: rows read once and written once, 4 B a sample"}
+                "note": "FP32 FFT filter: rows read once and written once, 4 B a sample, against the HBM copy bandwidth; "
+                        "what bounds it is shared-memory wavefronts (67 %) and issue (63 %), "
+                        "profiles/k_filter_fft_rows64_short.md"}
     else:
         flop = 2.0 * rows * d.n_channels * d.n_channels
         fpk = SMS * 128 * 2 * mhz * 1e6 / 1e12

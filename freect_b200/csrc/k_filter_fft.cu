@@ -44,6 +44,10 @@
 // is two radix-8 transforms. Real and imaginary parts are separate arrays with
 // a pad of R3 words per k1 block and the 16-byte chunks of a radix-R3 group
 // permuted, which makes every access of the five passes conflict-free.
+//
+// Bound by shared-memory wavefronts (67 % of the pipe) and issue (63 %) at 16 warps
+// per SM, by registers: 64 rows of 888 channels, 2460 views, 0.83 ms (Toeplitz
+// product 5.8).
 #include "wfbp_internal.h"
 
 #include <math.h>
